@@ -23,7 +23,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 SOURCES_CU = ["dgpu_kernels.cu"]
 SOURCES_CPP = ["dgpu_host.cpp", "dgpu_service.cpp", "dgpu_derep.cpp", "dgpu_errfun.cpp", "dgpu_errfun_external.cpp"]
-HEADERS = ["dgpu_common.h"]
+HEADERS = ["dgpu_common.h", "dgpu_strip.cuh"]
 
 
 def _stale(target: str, deps: list[str]) -> bool:

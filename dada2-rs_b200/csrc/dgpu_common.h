@@ -105,14 +105,17 @@ struct NwGeom {
   size_t vec_scratch;  // bytes per warp (pointer matrix)
   size_t rm_scratch;   // bytes per warp (pointer bit planes)
   int32_t forms;       // the aligner forms a compare launch can reach (kForms*)
+  int32_t strip_c;     // strip aligner: diagonals per strip of the widest pair (1..4; 0: not used)
+  int32_t strip_smem;  // its pointer words stay in shared memory
 };
 // Aligner forms a compare launch can reach, fixed by the pool's geometry and
 // parameters; k_align is compiled once per set, so a launch runs only the code
 // it can use (a smaller kernel: fewer instruction-cache misses in the
 // latency-bound late calls, and no register pressure from unused forms).
 constexpr int32_t kFormsAll = 0;   // every form
-constexpr int32_t kFormsVec1 = 1;  // gapless and the fast register form with one lane group
+constexpr int32_t kFormsStrip1 = 1;  // gapless and the strip aligner, one diagonal per strip, no homopolymer gaps
 constexpr int32_t kFormsRm = 2;    // gapless and the row-major forms
+constexpr int32_t kFormsStrip = 3;   // gapless and the strip aligner, up to four diagonals per strip
 
 // ---- shared-memory carving, used by kernels and by the host sizing code ----
 constexpr int kScreenWarps = 8;   // warps per screen CTA
@@ -120,6 +123,9 @@ constexpr int kScreenSmemTasks = 128; // tasks whose table the screen keeps in s
 constexpr int kNwWarps = 4;       // warps per NW CTA
 constexpr int kAlignCtasPerSm = 4; // resident align CTAs per SM (128 registers per thread)
 constexpr int kStageBytes = 4096; // traceback staging per warp
+constexpr int kStripPad = 16;     // readable bytes past the strip aligner's staged sequences
+constexpr int kStripWindow = 16;  // 256-byte rows of pointer words its traceback stages at once
+constexpr size_t kStripSmemMax = 8192;  // pointer words of a pair kept in shared memory up to this size
 constexpr uint32_t kNoPivot = 0xffffffffu;
 constexpr int kRmStageRows = 128; // anti-diagonals of pointer planes the row-major traceback stages at once
 constexpr int kStoreSpan = 2048;  // raws per store CTA (its own output segment)
@@ -152,12 +158,42 @@ __host__ __device__ inline size_t nw_smem_per_warp_rm(const NwGeom& g) {
   return align16(g.lmax) * 2 + rm_stage_bytes(kb) + align16(g.lmax) +
          (rm_fidx_in_stage(g.lmax, kb) ? 0 : align16(size_t(g.lmax) * 2));
 }
+// Diagonals per strip for bands of W diagonals: 31 lanes of two strips hold
+// them, and the lane after the last one in use holds the mark outside the band.
+__host__ __device__ inline int strip_cols(int64_t W) { return int((W + 61) / 62); }
+// Whether the strip aligner takes every pair of sequences of 2..lmax bases
+// with at most W diagonals. It reproduces the vectorized and the row-major
+// aligners' moves (vec: the pair takes the vectorized one) as long as no gap
+// scores above 0, no value comes near the marks these put outside the band
+// (-9999 and about -32760; a value is never below a run of mismatches along its
+// diagonal) and none saturates 16 bits where the vectorized one works in them.
+__host__ __device__ inline bool strip_takes(int64_t lmax, int64_t W, bool vec, int match, int mismatch, int gap,
+                                            int homo_gap) {
+  const int64_t up = match > mismatch ? match : mismatch, low = mismatch < match ? mismatch : match;
+  if (gap > 0 || homo_gap > 0 || gap < -1000 || homo_gap < -1000 || up > 1000 || low < -1000) return false;
+  if (W > 4 * 62 || -low * lmax > (vec ? 30000 : 9990)) return false;
+  return !vec || up * (lmax + 1) <= 32767;
+}
+__host__ __device__ inline size_t strip_plane_bytes(int64_t lmax, int c) {
+  return size_t((lmax + 32 + 2 * c) / (32 / (2 * c)) + 2) * 256;
+}
+__host__ __device__ inline size_t strip_smem_per_warp(const NwGeom& g) {
+  const size_t st = g.strip_smem ? strip_plane_bytes(g.lmax, g.strip_c) : size_t(kStripWindow) * 256;
+  const size_t fi = align16(size_t(g.lmax) * 2);
+  return 2 * align16(size_t(g.lmax) + kStripPad) + 2 * align16(size_t(g.lmax)) + (st > fi ? st : fi);
+}
+// Bytes of global scratch an alignment warp needs.
+__host__ __device__ inline size_t nw_scratch_bytes(const NwGeom& g) {
+  if (g.strip_c) return g.strip_smem ? 0 : strip_plane_bytes(g.lmax, g.strip_c);
+  return g.vec_scratch > g.rm_scratch ? g.vec_scratch : g.rm_scratch;
+}
 // The align kernel carves either layout from the same per-warp region, sized
 // for the forms the geometry lets a pair take (a zero scratch size marks a
 // form no pair of the launch can reach: the register form needs a vectorized
 // launch without homopolymer gaps and both lengths <= 3500; every other pair
 // is row-major).
 __host__ __device__ inline size_t align_smem_per_warp(const NwGeom& g) {
+  if (g.strip_c) return strip_smem_per_warp(g);
   const size_t a = g.vec_scratch ? nw_smem_per_warp_vec(g) : 0, b = g.rm_scratch ? nw_smem_per_warp_rm(g) : 0;
   const size_t m = a > b ? a : b;
   return m > 16 ? m : 16;
@@ -195,7 +231,7 @@ struct CompareLaunch {
   uint32_t* queue_pass;     // nraw capacity: items that passed the screen
   uint32_t* queue_counts;   // 8 words; [4] = items pushed to queue_pass, [5] = profiles the
                             // screen read, [6] = the align warps' slot cursor
-  uint8_t* nw_scratch;      // nwarps * max(vec_scratch, rm_scratch)
+  uint8_t* nw_scratch;      // nwarps * nw_scratch_bytes(geom)
   NwGeom geom;
   uint32_t* err_word;
   // store outputs

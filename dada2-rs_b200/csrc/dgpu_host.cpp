@@ -768,17 +768,17 @@ struct Pool {
     geom.vec_scratch = vec_possible ? align16(size_t(geom.vec_nrow) * std::max<size_t>(size_t(geom.vec_ncol), 32)) : 0;
     geom.rm_scratch = rm_possible ? align16(size_t(2 * lmax + 1) * 2 * kb * 4) : 0;
     geom.nwarps = sms * tuning_for(lmax).align_ctas_per_sm * kNwWarps;
-    // the forms k_align can reach (vec_align_any takes the fast register form
-    // with one lane group for every pair when the compressed width is <= 32,
-    // gaps are not positive and no sum can saturate i16)
-    geom.forms = kFormsAll;
-    if (rm_possible && !vec_possible) {
-      geom.forms = kFormsRm;
-    } else if (vec_possible && !rm_possible) {
-      const int64_t pmax = std::max<int64_t>({int64_t(kp.match), int64_t(kp.mismatch), 0});
-      if (geom.vec_ncol <= 32 && kp.gap <= 0 && pmax * (int64_t(lmax) + 1) <= 32767) geom.forms = kFormsVec1;
+    // the forms k_align can reach: the strip aligner alone when it takes every
+    // pair (see strip_takes), one diagonal per strip when no pair needs more
+    geom.forms = rm_possible && !vec_possible ? kFormsRm : kFormsAll;
+    geom.strip_c = geom.strip_smem = 0;
+    if (rm_possible != vec_possible &&
+        strip_takes(lmax, W, vec_possible, kp.match, kp.mismatch, kp.gap, use_homo ? kp.homo_gap : kp.gap)) {
+      geom.strip_c = strip_cols(W);
+      geom.strip_smem = strip_plane_bytes(lmax, geom.strip_c) <= kStripSmemMax ? 1 : 0;
+      geom.forms = geom.strip_c == 1 && !use_homo ? kFormsStrip1 : kFormsStrip;
     }
-    const size_t per = std::max<size_t>(std::max(geom.vec_scratch, geom.rm_scratch), 16);
+    const size_t per = std::max<size_t>(nw_scratch_bytes(geom), 16);
     slots.clear();
     for (int k = 0; k < nslots; ++k) {
       slots.emplace_back(new Slot);
@@ -4072,7 +4072,12 @@ int dgpu_align_debug(int device, int which, int npairs, const uint8_t* s1cat, co
   g.vec_scratch = align16(size_t(g.vec_nrow) * std::max<size_t>(size_t(g.vec_ncol), 32));
   g.rm_scratch = align16(size_t(2 * lmax + 1) * 2 * rm_kbound(g.rm_pairs) * 4);
   g.nwarps = npairs;
-  const size_t per = which == 0 ? g.vec_scratch : g.rm_scratch;
+  if (lmin >= 2 && end_gap == 0 &&
+      strip_takes(lmax, W, which == 0, kp.match, kp.mismatch, kp.gap, which == 1 ? kp.homo_gap : kp.gap)) {
+    g.strip_c = strip_cols(W);
+    g.strip_smem = strip_plane_bytes(lmax, g.strip_c) <= kStripSmemMax ? 1 : 0;
+  }
+  const size_t per = g.strip_c ? strip_plane_bytes(lmax, g.strip_c) : (which == 0 ? g.vec_scratch : g.rm_scratch);
   DBuf<uint8_t> d1, d2, scr, a0, a1;
   DBuf<uint32_t> o1, l1, o2, l2, ao, al, ew;
   TRY(d1.alloc(b1));

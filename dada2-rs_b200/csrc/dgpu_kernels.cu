@@ -208,6 +208,12 @@ void launch_fill_f64(double* p, size_t n, double v, cudaStream_t st) {
 // of the transition counts).
 constexpr unsigned kUnaligned = 0x80u;
 
+}  // namespace dgpu
+
+#include "dgpu_strip.cuh"
+
+namespace dgpu {
+
 // fidx[p] = err row * ncol + quality column for raw position p; lane 0 then forms
 // the left-to-right product (src/pval.rs:311-313). Returns the product on all lanes.
 __device__ double lambda_chain(int lane, const uint16_t* fidx, int L, const double* err_s) {
@@ -1736,10 +1742,6 @@ __device__ bool vec_align_fast(int lane, int len1, int len2, int match, int mism
 // Picks the register form when the pair's compressed width fits 128 columns.
 // With `staged` the caller has already put the shorter sequence (the first on
 // ties) in S.s1 and the other in S.s2, and g1/g2 point at those copies.
-// ONLY_M1: the caller has shown that every pair takes the fast form with one
-// lane group (kFormsVec1); the other forms are not compiled in, and a pair
-// outside it is refused.
-template <bool ONLY_M1 = false>
 __device__ bool vec_align_any(int lane, const uint8_t* g1, int l1, const uint8_t* g2, int l2, int16_t match,
                               int16_t mismatch, int16_t gap, int16_t egp, int band_in, const VecSmem& S,
                               uint8_t* scratch, int ncol_bound, int nrow_bound, uint32_t* ham_out, uint32_t* err_word,
@@ -1753,10 +1755,6 @@ __device__ bool vec_align_any(int lane, const uint8_t* g1, int l1, const uint8_t
   const int pmax = max(max(int(match), int(mismatch)), 0);
   const bool fast = ncol >= 4 && ncol <= 128 && len1 >= 1 && nrow <= nrow_bound && gap <= 0 && egp <= 0 &&
                     pmax * ((len1 + len2) / 2 + 1) <= 32767;
-  if (ONLY_M1 && !(fast && ncol <= 32)) {
-    if (lane == 0) atomicOr(err_word, DERR_UNSUPPORTED);
-    return false;
-  }
   if (fast) {
     const bool swap = l1 > l2;
     {
@@ -1785,17 +1783,14 @@ __device__ bool vec_align_any(int lane, const uint8_t* g1, int l1, const uint8_t
       if (swap) VEC_FAST(1, true);
       VEC_FAST(1, false);
     }
-    if constexpr (!ONLY_M1) {
-      if (mw == 2) {
-        if (swap) VEC_FAST(2, true);
-        VEC_FAST(2, false);
-      }
-      if (swap) VEC_FAST(4, true);
-      VEC_FAST(4, false);
+    if (mw == 2) {
+      if (swap) VEC_FAST(2, true);
+      VEC_FAST(2, false);
     }
+    if (swap) VEC_FAST(4, true);
+    VEC_FAST(4, false);
 #undef VEC_FAST
   }
-  if constexpr (ONLY_M1) return false;  // not reached: refused above
   if (ncol <= 32)
     return vec_align_reg<1>(lane, g1, l1, g2, l2, match, mismatch, gap, egp, band_in, S, w, nrow_bound, ham_out,
                             err_word, dbg0, dbg1, dbg_len);
@@ -2375,6 +2370,81 @@ struct PairResult {
   const uint8_t* qual;
 };
 
+// Whether the pair takes the gapless alignment (src/nwalign.rs:1324-1403): the
+// ordered k-mer distance (src/kmers.rs:314-328) equals the screen's, or the
+// band is 0. *ham then holds the mismatches of the shared length.
+__device__ __forceinline__ bool takes_gapless(int lane, const KParams& kp, const uint8_t* sc, int lc,
+                                              const uint8_t* sg, int lg, double kdist, uint32_t* ham) {
+  const int k = kp.kmer_size;
+  double kodist = -1.0;
+  const int minl = lc < lg ? lc : lg;
+  const bool want_kod = kp.use_kmers && kp.gapless && lc == lg;
+  if (want_kod || kp.band == 0) {
+    const int klen = lc - (k - 1);
+    const uint32_t kmask = (k >= 32) ? 0xffffffffu : ((1u << k) - 1u);
+    uint32_t eq = 0, mm = 0;
+    uint32_t cur = mismatch_word(sc, sg, 0, minl, lane);
+    for (int b = 0; b < minl; b += 32) {
+      const uint32_t nxt = mismatch_word(sc, sg, b + 32, minl, lane);
+      mm += __popc(cur);
+      if (want_kod) {
+        const unsigned long long both = (static_cast<unsigned long long>(nxt) << 32) | cur;
+        const int j = b + lane;
+        const bool ok = j < klen && ((uint32_t(both >> lane) & kmask) == 0u);
+        eq += __popc(__ballot_sync(FULL, ok));
+      }
+      cur = nxt;
+    }
+    *ham = mm;
+    if (want_kod && klen > 0) kodist = 1.0 - double(eq) / double(klen);
+  }
+  return kp.band == 0 || (kp.gapless && fabs(kodist - kdist) < DBL_EPSILON);
+}
+
+// The gapless alignment's rows: raw position p aligns to center position p
+// while p < len(center).
+__device__ __forceinline__ void gapless_codes(int lane, const uint8_t* sc, int lc, const uint8_t* sg, int lg,
+                                              uint8_t* tcode) {
+  for (int p = lane; p < lg; p += 32) {
+    const unsigned r = sg[p];
+    const unsigned code = (p < lc) ? (unsigned(sc[p]) - 1u) * 4u + (r - 1u) : (kUnaligned | ((r - 1u) * 5u));
+    const bool valid = r >= 1u && r <= 4u && (p >= lc || (sc[p] >= 1 && sc[p] <= 4));
+    tcode[p] = uint8_t(valid ? code : 255u);
+  }
+}
+
+// align_pair for launches whose geometry lets every pair take the strip
+// aligner (NwGeom::strip_c). planes: the warp's pointer words in global memory
+// when they do not stay in shared memory.
+template <int FORMS>
+__device__ __forceinline__ PairResult align_pair_strip(int lane, const KParams& kp, const PoolDev& pool,
+                                                       const NwGeom& geom, uint32_t g, uint32_t c, double kdist,
+                                                       bool want_qual, const StripSmem& S, uint8_t* scratch,
+                                                       uint32_t* err_word) {
+  const int lc = int(pool.len[c]), lg = int(pool.len[g]);
+  const uint8_t* qg = pool.qual ? pool.qual + pool.off[g] : nullptr;
+  const bool stage_q = want_qual && qg != nullptr;
+  stage3(lane, pool.seq + pool.off[c], lc, S.s1, pool.seq + pool.off[g], lg, S.s2, stage_q ? qg : nullptr, S.qual);
+  __syncwarp();
+  PairResult R{true, AM_NONE, 0u, lg, S.tcode, S.fidx, stage_q ? S.qual : qg};
+  uint32_t ham = 0;
+  if (takes_gapless(lane, kp, S.s1, lc, S.s2, lg, kdist, &ham)) {
+    gapless_codes(lane, S.s1, lc, S.s2, lg, S.tcode);
+    R.method = AM_GAPLESS;
+  } else {
+    const bool homo = FORMS != kFormsStrip1 && kp.homo_gap != kp.gap && kp.homo_gap <= 0;
+    const bool in_smem = geom.strip_smem != 0;
+    uint2* planes = in_smem ? S.stage : reinterpret_cast<uint2*>(scratch);
+    constexpr int CMAX = FORMS == kFormsStrip1 ? 1 : 4;
+    R.ok = strip_dispatch<CMAX, FORMS != kFormsStrip1>(lane, lc, lg, kp, homo, S, planes, in_smem, &ham, err_word,
+                                                       nullptr, nullptr, nullptr);
+    R.method = homo ? AM_HOMO : ((kp.vectorized && lc <= 3500 && lg <= 3500) ? AM_VECTORIZED : AM_ENDSFREE);
+  }
+  R.ham = ham;
+  __syncwarp();
+  return R;
+}
+
 // COOP: every warp of the CTA calls this with the same pair and warp 0's
 // buffers (VS, RS, scratch); the row-major DP is shared (rm_dispatch_coop),
 // everything else is warp 0's, and only warp 0's result is meaningful. It is
@@ -2387,14 +2457,13 @@ __device__ __forceinline__ PairResult align_pair(int lane, const KParams& kp, co
                                                  uint32_t g, uint32_t c, double kdist, bool want_qual,
                                                  const VecSmem& VS, const RmSmem& RS, int kb, uint8_t* scratch,
                                                  uint32_t* err_word, int wib = 0, int* xch = nullptr) {
-  const int k = kp.kmer_size;
   const int lc = int(pool.len[c]), lg = int(pool.len[g]);
   const uint8_t* sc = pool.seq + pool.off[c];
   const uint8_t* sg = pool.seq + pool.off[g];
   const uint8_t* qg = pool.qual ? pool.qual + pool.off[g] : nullptr;
   const bool use_homo = kp.homo_gap != kp.gap && kp.homo_gap <= 0;
   const bool rm_pair = use_homo || !kp.vectorized || lc > 3500 || lg > 3500;
-  const bool rm = FORMS == kFormsRm ? true : (FORMS == kFormsVec1 ? false : rm_pair);
+  const bool rm = FORMS == kFormsRm ? true : rm_pair;
   if (rm != rm_pair) {
     if (lane == 0) atomicOr(err_word, DERR_UNSUPPORTED);
     return PairResult{false, AM_NONE, 0u, lg, VS.tcode, VS.fidx, qg};
@@ -2411,57 +2480,26 @@ __device__ __forceinline__ PairResult align_pair(int lane, const KParams& kp, co
     sg = dg;
     if (stage_q) qg = dq;
   }
-  double kodist = -1.0;
-  const int minl = lc < lg ? lc : lg;
-  const bool want_kod = kp.use_kmers && kp.gapless && lc == lg;
   // the raw's transition codes and lambda indices live in the layout of the
   // form this pair takes (the per-warp region holds only the forms the
   // launch can reach)
   PairResult R{true, AM_NONE, 0u, lg, rm ? RS.tcode : VS.tcode, rm ? RS.fidx : VS.fidx, qg};
   uint32_t ham = 0;
-  if (want_kod || kp.band == 0) {
-    const int klen = lc - (k - 1);
-    const uint32_t kmask = (k >= 32) ? 0xffffffffu : ((1u << k) - 1u);
-    uint32_t eq = 0;
-    uint32_t cur = mismatch_word(sc, sg, 0, minl, lane);
-    for (int b = 0; b < minl; b += 32) {
-      const uint32_t nxt = mismatch_word(sc, sg, b + 32, minl, lane);
-      ham += __popc(cur);
-      if (want_kod) {
-        const unsigned long long both = (static_cast<unsigned long long>(nxt) << 32) | cur;
-        const int j = b + lane;
-        const bool ok = j < klen && ((uint32_t(both >> lane) & kmask) == 0u);
-        eq += __popc(__ballot_sync(FULL, ok));
-      }
-      cur = nxt;
-    }
-    if (want_kod && klen > 0) kodist = 1.0 - double(eq) / double(klen);
-  }
-  const bool gapless = kp.band == 0 || (kp.gapless && fabs(kodist - kdist) < DBL_EPSILON);
+  const bool gapless = takes_gapless(lane, kp, sc, lc, sg, lg, kdist, &ham);
   if (gapless) {
-    // raw position p aligns to center position p while p < len(center)
-    uint8_t* tcode = rm ? RS.tcode : VS.tcode;
-    for (int p = (!COOP || wib == 0) ? lane : lg; p < lg; p += 32) {
-      const unsigned r = sg[p];
-      const unsigned code = (p < lc) ? (unsigned(sc[p]) - 1u) * 4u + (r - 1u) : (kUnaligned | ((r - 1u) * 5u));
-      const bool valid = r >= 1u && r <= 4u && (p >= lc || (sc[p] >= 1 && sc[p] <= 4));
-      tcode[p] = uint8_t(valid ? code : 255u);
-    }
+    if (!COOP || wib == 0) gapless_codes(lane, sc, lc, sg, lg, rm ? RS.tcode : VS.tcode);
     R.method = AM_GAPLESS;
   } else if (!COOP && !rm) {
-    R.ok = vec_align_any<FORMS == kFormsVec1>(lane, sc, lc, sg, lg, int16_t(kp.match), int16_t(kp.mismatch),
-                                              int16_t(kp.gap), 0, kp.band,
+    R.ok = vec_align_any(lane, sc, lc, sg, lg, int16_t(kp.match), int16_t(kp.mismatch), int16_t(kp.gap), 0, kp.band,
                          VS, scratch, geom.vec_ncol, geom.vec_nrow, &ham, err_word, nullptr, nullptr, nullptr, true);
     R.method = AM_VECTORIZED;
   } else {
-    if constexpr (FORMS != kFormsVec1) {
-      if (COOP)
-        R.ok = rm_dispatch_coop(lane, wib, sc, lc, sg, lg, kp, use_homo, kb, RS, reinterpret_cast<uint32_t*>(scratch),
-                                &ham, err_word, xch);
-      else
-        R.ok = rm_dispatch(lane, sc, lc, sg, lg, kp, use_homo, kb, RS, reinterpret_cast<uint32_t*>(scratch), &ham,
-                           err_word, nullptr, nullptr, nullptr);
-    }
+    if (COOP)
+      R.ok = rm_dispatch_coop(lane, wib, sc, lc, sg, lg, kp, use_homo, kb, RS, reinterpret_cast<uint32_t*>(scratch),
+                              &ham, err_word, xch);
+    else
+      R.ok = rm_dispatch(lane, sc, lc, sg, lg, kp, use_homo, kb, RS, reinterpret_cast<uint32_t*>(scratch), &ham,
+                         err_word, nullptr, nullptr, nullptr);
     R.tcode = RS.tcode;
     R.fidx = RS.fidx;
     R.method = use_homo ? AM_HOMO : AM_ENDSFREE;
@@ -2495,16 +2533,14 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
   // four lane groups: the CTA's warps share each pair (rm_align_coop), which
   // cuts a long pair's latency, the bound of such calls. Wider bands (eight
   // or sixteen groups, G > 1 per warp) keep one warp per pair.
-  const bool coop = FORMS != kFormsVec1 && L.geom.vec_scratch == 0 && kb >= 2 && kb <= kNwWarps &&
-                    count <= 2u * gridDim.x;
+  constexpr bool STRIP = FORMS == kFormsStrip1 || FORMS == kFormsStrip;
+  const bool coop = !STRIP && L.geom.vec_scratch == 0 && kb >= 2 && kb <= kNwWarps && count <= 2u * gridDim.x;
   if (blockIdx.x * (coop ? 1u : uint32_t(kNwWarps)) >= count) return;  // nothing queued for this block
   const size_t err_bytes = err_smem_bytes(kp.ncol);
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int gw = blockIdx.x * kNwWarps + wib;
   unsigned char* wbase = smem_raw + err_bytes + size_t(wib) * align_smem_per_warp(L.geom);
-  const VecSmem VS = carve_vec(wbase, L.geom.lmax, L.geom.vec_ncol);
-  const RmSmem RS = carve_rm(wbase, L.geom.lmax, kb);
-  const size_t scr_stride = L.geom.vec_scratch > L.geom.rm_scratch ? L.geom.vec_scratch : L.geom.rm_scratch;
+  const size_t scr_stride = nw_scratch_bytes(L.geom);
   uint8_t* scratch = L.nw_scratch + size_t(gw) * scr_stride;
   __syncthreads();
   // lambda and the raw's result entries, by the warp that holds the alignment
@@ -2529,7 +2565,7 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
     }
     __syncwarp();
   };
-  if constexpr (FORMS != kFormsVec1) if (coop) {
+  if constexpr (!STRIP) if (coop) {
     // Thread 0 claims a slot for the CTA and reads the raw's screen distance
     // (which warp 0 overwrites with lambda when the pair is done) into shared
     // memory, so every warp takes the same branches through the pair and the
@@ -2575,18 +2611,32 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
   // against NW, short against long -- and CTAs that become resident late
   // (when shared memory admits fewer CTAs per SM than the grid assumes) even
   // out. Results go to each raw's own entries, so the order is free.
-  for (;;) {
-    uint32_t slot = 0;
-    if (lane == 0) slot = atomicAdd(&L.queue_counts[6], 1u);
-    slot = __shfl_sync(FULL, slot, 0);
-    if (slot >= count) break;
-    const uint32_t item = L.queue_pass[slot];
-    const uint32_t t = find_task(L.task_prefix, L.ntask, item);
-    const TaskDev T = L.tasks[t];
-    const uint32_t g = T.base + (item - L.task_prefix[t]);
-    const PairResult R = align_pair<false, FORMS>(lane, kp, L.pool, L.geom, g, T.center, L.pool.res_lambda[g],
-                                           kp.use_quals != 0, VS, RS, kb, scratch, L.err_word);
-    finish(R, g);
+  auto each_pair = [&](auto&& align) {
+    for (;;) {
+      uint32_t slot = 0;
+      if (lane == 0) slot = atomicAdd(&L.queue_counts[6], 1u);
+      slot = __shfl_sync(FULL, slot, 0);
+      if (slot >= count) break;
+      const uint32_t item = L.queue_pass[slot];
+      const uint32_t t = find_task(L.task_prefix, L.ntask, item);
+      const TaskDev T = L.tasks[t];
+      const uint32_t g = T.base + (item - L.task_prefix[t]);
+      finish(align(g, T.center), g);
+    }
+  };
+  if constexpr (STRIP) {
+    const StripSmem S = carve_strip(wbase, L.geom);
+    each_pair([&](uint32_t g, uint32_t c) {
+      return align_pair_strip<FORMS>(lane, kp, L.pool, L.geom, g, c, L.pool.res_lambda[g], kp.use_quals != 0, S,
+                                     scratch, L.err_word);
+    });
+  } else {
+    const VecSmem VS = carve_vec(wbase, L.geom.lmax, L.geom.vec_ncol);
+    const RmSmem RS = carve_rm(wbase, L.geom.lmax, kb);
+    each_pair([&](uint32_t g, uint32_t c) {
+      return align_pair<false, FORMS>(lane, kp, L.pool, L.geom, g, c, L.pool.res_lambda[g], kp.use_quals != 0, VS, RS,
+                                      kb, scratch, L.err_word);
+    });
   }
 }
 
@@ -2599,7 +2649,9 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
 // sample's 16 x tncol matrix. Warps take contiguous runs of items (ordered by
 // sample), count in a shared-memory histogram and flush it to the sample's
 // matrix when the sample changes and at the end.
+template <int FORMS>
 __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_final_subs(FinalSubsLaunch F) {
+  constexpr bool STRIP = FORMS == kFormsStrip1 || FORMS == kFormsStrip;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const KParams& kp = F.kp;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -2608,11 +2660,9 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_final_subs(F
   const int kb = rm_kbound(F.geom.rm_pairs);
   const size_t per_warp = align_smem_per_warp(F.geom) + align16(size_t(16) * F.tncol * 4);
   unsigned char* wbase = smem_raw + size_t(wib) * per_warp;
-  const VecSmem VS = carve_vec(wbase, F.geom.lmax, F.geom.vec_ncol);
-  const RmSmem RS = carve_rm(wbase, F.geom.lmax, kb);
   uint32_t* hist = reinterpret_cast<uint32_t*>(wbase + align_smem_per_warp(F.geom));
   const int nbins = 16 * F.tncol;
-  const size_t scr_stride = F.geom.vec_scratch > F.geom.rm_scratch ? F.geom.vec_scratch : F.geom.rm_scratch;
+  const size_t scr_stride = nw_scratch_bytes(F.geom);
   uint8_t* scratch = F.nw_scratch + size_t(gw) * scr_stride;
   for (int b = lane; b < nbins; b += 32) hist[b] = 0;
   __syncwarp();
@@ -2633,6 +2683,16 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_final_subs(F
     }
     __syncwarp();
   };
+  auto align_one = [&](uint32_t g, uint32_t c) {
+    if constexpr (STRIP) {
+      return align_pair_strip<FORMS>(lane, kp, F.pool, F.geom, g, c, 0.0, F.has_quals != 0, carve_strip(wbase, F.geom),
+                                     scratch, F.err_word);
+    } else {
+      return align_pair<false>(lane, kp, F.pool, F.geom, g, c, 0.0, F.has_quals != 0,
+                               carve_vec(wbase, F.geom.lmax, F.geom.vec_ncol), carve_rm(wbase, F.geom.lmax, kb), kb,
+                               scratch, F.err_word);
+    }
+  };
   uint64_t bound = 0;  // what the shared bins may hold since the last flush
   for (uint32_t i = i0; i < i1; ++i) {
     const uint32_t g = F.raw[i], c = F.center[i], smp = F.sample[i];
@@ -2646,8 +2706,7 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_final_subs(F
       bound = 0;
     }
     bound += add;
-    const PairResult R = align_pair<false>(lane, kp, F.pool, F.geom, g, c, 0.0, F.has_quals != 0, VS, RS, kb, scratch,
-                                    F.err_word);
+    const PairResult R = align_one(g, c);
     if (!R.ok) continue;  // the error word reports it
     const uint32_t reads = F.pool.reads[g];
     const bool direct = add > 0xffffffffull;  // alone it could wrap a 32-bit bin: count in global memory
@@ -2668,8 +2727,11 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_final_subs(F
 void launch_final_subs(const FinalSubsLaunch& F, cudaStream_t st) {
   if (F.nitems == 0) return;
   const size_t smem = size_t(kNwWarps) * (align_smem_per_warp(F.geom) + align16(size_t(16) * F.tncol * 4));
-  if (smem > 48 * 1024) cudaFuncSetAttribute(k_final_subs, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-  k_final_subs<<<F.geom.nwarps / kNwWarps, kNwWarps * 32, smem, st>>>(F);
+  void (*kern)(FinalSubsLaunch) = F.geom.forms == kFormsStrip1  ? k_final_subs<kFormsStrip1>
+                                  : F.geom.forms == kFormsStrip ? k_final_subs<kFormsStrip>
+                                                                : k_final_subs<kFormsAll>;
+  if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  kern<<<F.geom.nwarps / kNwWarps, kNwWarps * 32, smem, st>>>(F);
 }
 
 // ---------------------------------------------------------------------------
@@ -2855,12 +2917,12 @@ uint32_t compare_screen_chunk(uint32_t total, uint32_t screen_blocks_per_sm, uin
 // set once per device (dynamic shared memory above 48 KB, the largest
 // carveout so that kAlignCtasPerSm CTAs fit beside each other).
 static void (*align_kernel(const CompareLaunch& L, size_t smem))(CompareLaunch) {
-  void (*kalign)(CompareLaunch) = L.geom.forms == kFormsVec1 ? k_align<kFormsVec1>
-                                  : L.geom.forms == kFormsRm ? k_align<kFormsRm>
-                                                             : k_align<kFormsAll>;
-  const int fi = L.geom.forms == kFormsVec1 ? 1 : (L.geom.forms == kFormsRm ? 2 : 0);
-  static std::atomic<int> limit[3][64];
-  static std::atomic<uint64_t> carved[3];
+  static void (*const forms[4])(CompareLaunch) = {k_align<kFormsAll>, k_align<kFormsStrip1>, k_align<kFormsRm>,
+                                                  k_align<kFormsStrip>};
+  const int fi = L.geom.forms;
+  void (*kalign)(CompareLaunch) = forms[fi];
+  static std::atomic<int> limit[4][64];
+  static std::atomic<uint64_t> carved[4];
   int dev = 0;
   cudaGetDevice(&dev);
   std::atomic<int>& lim = limit[fi][dev & 63];
@@ -2974,12 +3036,22 @@ __global__ void __launch_bounds__(kNwWarps * 32) k_align_debug(int which, const 
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const uint32_t pair = blockIdx.x * kNwWarps + wib;
   if (pair >= npairs) return;
-  const size_t scr = which == 0 ? geom.vec_scratch : geom.rm_scratch;
+  const size_t scr = geom.strip_c ? strip_plane_bytes(geom.lmax, geom.strip_c)
+                                  : (which == 0 ? geom.vec_scratch : geom.rm_scratch);
   uint8_t* my_scr = scratch + size_t(pair) * scr;
   uint32_t ham = 0;
   const uint8_t* a = s1cat + off1[pair];
   const uint8_t* b = s2cat + off2[pair];
-  if (which == 0) {
+  if (geom.strip_c) {  // every pair takes the strip aligner, as the compare step's do
+    const int n1 = int(len1[pair]), n2 = int(len2[pair]);
+    const StripSmem S = carve_strip(smem_raw + size_t(wib) * strip_smem_per_warp(geom), geom);
+    for (int p = lane; p < n1; p += 32) S.s1[p] = a[p];
+    for (int p = lane; p < n2; p += 32) S.s2[p] = b[p];
+    __syncwarp();
+    uint2* planes = geom.strip_smem ? S.stage : reinterpret_cast<uint2*>(my_scr);
+    strip_dispatch<4, true>(lane, n1, n2, kp, which == 1, S, planes, geom.strip_smem != 0, &ham, err_word,
+                            al0 + aloff[pair], al1 + aloff[pair], alen + pair);
+  } else if (which == 0) {
     VecSmem S = carve_vec(smem_raw + size_t(wib) * nw_smem_per_warp_vec(geom), geom.lmax, geom.vec_ncol);
     vec_align_any(lane, a, int(len1[pair]), b, int(len2[pair]), int16_t(kp.match), int16_t(kp.mismatch),
                   int16_t(kp.gap), int16_t(end_gap), kp.band, S, my_scr, geom.vec_ncol, geom.vec_nrow, &ham, err_word,
@@ -2997,7 +3069,8 @@ void launch_align_debug(int which, const uint8_t* s1cat, const uint32_t* off1, c
                         int end_gap, const NwGeom& geom, uint8_t* scratch, uint8_t* al0, uint8_t* al1,
                         const uint32_t* aloff, uint32_t* alen, uint32_t* err_word, cudaStream_t st) {
   if (npairs == 0) return;
-  const size_t per = which == 0 ? nw_smem_per_warp_vec(geom) : nw_smem_per_warp_rm(geom);
+  const size_t per = geom.strip_c ? strip_smem_per_warp(geom)
+                                  : (which == 0 ? nw_smem_per_warp_vec(geom) : nw_smem_per_warp_rm(geom));
   const size_t smem = per * kNwWarps;
   if (smem > 48 * 1024) cudaFuncSetAttribute(k_align_debug, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   const uint32_t blocks = (npairs + kNwWarps - 1) / kNwWarps;
