@@ -124,7 +124,6 @@ constexpr int kNwWarps = 4;       // warps per NW CTA
 constexpr int kAlignCtasPerSm = 4; // resident align CTAs per SM (128 registers per thread)
 constexpr int kStageBytes = 4096; // traceback staging per warp
 constexpr int kStripPad = 16;     // readable bytes past the strip aligner's staged sequences
-constexpr int kStripWindow = 16;  // 256-byte rows of pointer words its traceback stages at once
 constexpr size_t kStripSmemMax = 8192;  // pointer words of a pair kept in shared memory up to this size
 constexpr uint32_t kNoPivot = 0xffffffffu;
 constexpr int kRmStageRows = 128; // anti-diagonals of pointer planes the row-major traceback stages at once
@@ -174,11 +173,13 @@ __host__ __device__ inline bool strip_takes(int64_t lmax, int64_t W, bool vec, i
   if (W > 4 * 62 || -low * lmax > (vec ? 30000 : 9990)) return false;
   return !vec || up * (lmax + 1) <= 32767;
 }
+// Rows whose pointer bits share one word (a power of two).
+__host__ __device__ constexpr int strip_rows_per_word(int c) { return c == 1 ? 16 : (c == 2 ? 8 : 4); }
 __host__ __device__ inline size_t strip_plane_bytes(int64_t lmax, int c) {
-  return size_t((lmax + 32 + 2 * c) / (32 / (2 * c)) + 2) * 256;
+  return size_t((lmax + 32 + 2 * c) / strip_rows_per_word(c) + 2) * 256;
 }
 __host__ __device__ inline size_t strip_smem_per_warp(const NwGeom& g) {
-  const size_t st = g.strip_smem ? strip_plane_bytes(g.lmax, g.strip_c) : size_t(kStripWindow) * 256;
+  const size_t st = g.strip_smem ? strip_plane_bytes(g.lmax, g.strip_c) : 0;
   const size_t fi = align16(size_t(g.lmax) * 2);
   return 2 * align16(size_t(g.lmax) + kStripPad) + 2 * align16(size_t(g.lmax)) + (st > fi ? st : fi);
 }

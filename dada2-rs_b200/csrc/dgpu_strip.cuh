@@ -18,7 +18,7 @@ struct StripSmem {
   uint8_t* s2;      // raw codes
   uint8_t* qual;    // raw qualities
   uint8_t* tcode;   // per raw position: error-matrix row (see kUnaligned)
-  uint2* stage;     // pointer words: all of them, or the traceback's window
+  uint2* stage;     // the pointer words, when they stay in shared memory
   uint16_t* fidx;   // in stage, which is free after the traceback
 };
 
@@ -56,84 +56,115 @@ __device__ __forceinline__ void band_offsets(int band, int len1, int len2, int* 
   }
 }
 
-// Walks the pointer words back from (len1, len2). Lane t tests whether the
-// t-th step back is diagonal (the same diagonal, row i - t), so a run of
-// diagonal steps and the gap that ends it are taken at once.
-template <int C>
+// Walks the pointer words back from (len1, len2). Lane t holds the words of
+// row i - t of the lane's diagonals that the walk is on; two ballots turn the
+// current diagonal's bits of the 32 rows into a run of diagonal steps and the
+// gap that ends it, until the walk leaves the rows or the diagonals. The next
+// 32 rows' words are on their way meanwhile. The bound is the chain of
+// dependent instructions of one warp, about 200 cycles a run: a walk that also
+// read its words anew for every run took 212,000 cycles for two unrelated
+// 1,450-nt sequences (345 runs) and 34,000 for two copies of one.
+template <int C, bool DBG>
 __device__ __forceinline__ bool strip_traceback(int lane, int len1, int len2, int o_lo, int W, const StripSmem& S,
-                                                const uint2* planes, bool in_smem, uint32_t* ham_out,
-                                                uint32_t* err_word, uint8_t* dbg0, uint8_t* dbg1, uint32_t* dbg_len) {
-  constexpr int N = 2 * C, RPW = 32 / N, NB = RPW * N;
-  for (int p = lane; p < len2; p += 32) S.tcode[p] = uint8_t(kUnaligned | (((S.s2[p] & 15u) - 1u) * 5u));
+                                                const uint2* planes, uint32_t* ham_out, uint32_t* err_word,
+                                                uint8_t* dbg0, uint8_t* dbg1, uint32_t* dbg_len) {
+  constexpr int N = 2 * C;
+  constexpr unsigned RPW = strip_rows_per_word(C), NB = RPW * N;
+  const uint8_t* const s1 = S.s1;
+  const uint8_t* const s2 = S.s2;
+  uint8_t* const tcode = S.tcode;
+  for (int p = lane; p < len2; p += 32) tcode[p] = uint8_t(kUnaligned | (((s2[p] & 15u) - 1u) * 5u));
   __syncwarp();
-  int i = len1, j = len2, slo = in_smem ? 0 : 0x7fffffff;
-  uint32_t ham = 0, alen = 0;
+  int i = len1, j = len2;
+  uint32_t mism = 0, alen = 0;
+  // rows count as the DP inserted them: row i of lane l is its (i + l - 1)-th
+  auto word_at = [&](int row, int l) -> uint2 {
+    const unsigned r = unsigned(max(row, 1) + l - 1);
+    return planes[(r / RPW) * 32 + l];
+  };
+  auto shift_of = [](int row, int l) -> unsigned { return NB - 1 - (unsigned(row + l - 1) % RPW) * N; };
+  // The free gaps of the last row or column are the one place of long gap
+  // runs: lane t tests the t-th next gap.
+  const bool longer2 = len2 > len1;
+  for (int g = 32; g == 32;) {
+    const int it = longer2 ? i : i - lane, jt = longer2 ? j - lane : j, xt = jt - it - o_lo;
+    bool same = it > 0 && jt > 0 && xt >= 0 && xt < W;
+    if (same) {
+      const int lt = xt / N;
+      const uint2 v = word_at(it, lt);
+      const unsigned b = shift_of(it, lt) - unsigned(xt - lt * N);
+      same = !((v.x >> b) & 1u) && bool((v.y >> b) & 1u) == longer2;
+    }
+    g = __clz(__brev(~__ballot_sync(FULL, same)));
+    if (DBG) {
+      if (lane < g) {
+        dbg0[alen + lane] = longer2 ? uint8_t('-') : uint8_t(s1[i - 1 - lane] & 15u);
+        dbg1[alen + lane] = longer2 ? uint8_t(s2[j - 1 - lane] & 15u) : uint8_t('-');
+      }
+      alen += uint32_t(g);
+    }
+    i -= longer2 ? 0 : g;
+    j -= longer2 ? g : 0;
+  }
+  uint2 wn = make_uint2(0u, 0u);
+  int wn_l = -1, wn_i = 0;  // wn: the words of rows wn_i .. wn_i - 31 of lane wn_l
+  bool bad = false;
   while (i > 0 && j > 0) {
     const int idx = j - i - o_lo;
-    if (idx < 0 || idx >= W) {
-      if (lane == 0) atomicOr(err_word, DERR_TRACEBACK);
-      return false;
-    }
-    const int l = idx / N, k = idx - l * N;
-    const int r = i + l - 1;
-    if (!in_smem && (r / RPW < slo || (slo > 0 && r - slo * RPW < 31))) {  // stage the next words down
-      const int hi = r / RPW, lo = max(0, hi - (kStripWindow - 1));
-      __syncwarp();
-      const uint4* src = reinterpret_cast<const uint4*>(planes + size_t(lo) * 32);
-      uint4* dst = reinterpret_cast<uint4*>(S.stage);
-      const int nv = (hi - lo + 1) * 16;
-#pragma unroll 4
-      for (int x = lane; x < nv; x += 32) dst[x] = __ldcg(src + x);
-      __syncwarp();
-      slo = lo;
-    }
-    const int rt = r - lane;  // the row this lane tests, as an insertion row
-    const bool ok = lane < i && lane < j && rt >= slo * RPW;
-    uint2 w = make_uint2(0u, 0u);
-    int bit = 0;
-    if (ok) {
-      const int wt = rt / RPW;
-      w = S.stage[(wt - slo) * 32 + l];
-      bit = NB - 1 - ((rt - wt * RPW) * N + k);
-    }
-    const bool diag = ok && ((w.x >> bit) & 1u);
-    const uint32_t nd = __ballot_sync(FULL, !diag);
-    const int f = nd ? __ffs(nd) - 1 : 32;
-    bool mm = false;
-    if (lane < f) {
-      const uint8_t a = S.s1[i - 1 - lane] & 15u, b = S.s2[j - 1 - lane] & 15u;
-      S.tcode[j - 1 - lane] = uint8_t((unsigned(a) - 1u) * 4u + (unsigned(b) - 1u));
-      mm = a != b;
-      if (dbg0) {
-        dbg0[alen + lane] = a;
-        dbg1[alen + lane] = b;
+    bad = unsigned(idx) >= unsigned(W);
+    if (bad) break;
+    const int l = idx / N, it = i - lane;
+    const uint2 w = wn_l == l && wn_i == i ? wn : word_at(it, l);
+    wn = word_at(it - 32, l);
+    wn_l = l;
+    wn_i = i - 32;
+    const unsigned sh = shift_of(it, l);
+    const unsigned a = s1[max(it - 1, 0)] & 15u;
+    int k = idx - l * N, t0 = 0;
+    do {
+      const unsigned b = (sh - unsigned(k)) & 31u;
+      const uint32_t d = __ballot_sync(FULL, (w.x >> b) & 1u), lf = __ballot_sync(FULL, (w.y >> b) & 1u);
+      const int f = min(__clz(__brev(~(d >> t0))), min(i, j));
+      const int u = lane - t0;
+      if (unsigned(u) < unsigned(f)) {
+        const unsigned c = s2[j - 1 - u] & 15u;
+        tcode[j - 1 - u] = uint8_t((a - 1u) * 4u + (c - 1u));
+        mism += a != c ? 1u : 0u;
+        if (DBG) {
+          dbg0[alen + u] = uint8_t(a);
+          dbg1[alen + u] = uint8_t(c);
+        }
       }
-    }
-    ham += __popc(__ballot_sync(FULL, mm));
-    // the step after the run, where its lane holds it: 1 left, 0 up, -1 not known
-    const int gap = __shfl_sync(FULL, ok ? int((w.y >> bit) & 1u) : -1, f & 31);
-    i -= f;
-    j -= f;
-    alen += uint32_t(f);
-    if (f < 32 && gap >= 0) {
-      if (gap) {
-        if (dbg0 && lane == 0) { dbg0[alen] = '-'; dbg1[alen] = S.s2[j - 1] & 15u; }
-        --j;
-      } else {
-        if (dbg0 && lane == 0) { dbg0[alen] = S.s1[i - 1] & 15u; dbg1[alen] = '-'; }
-        --i;
+      if (DBG) alen += uint32_t(f);
+      i -= f;
+      j -= f;
+      t0 += f;
+      if (t0 >= 32 || min(i, j) == 0) break;
+      const int left = int((lf >> t0) & 1u);
+      if (DBG) {
+        if (lane == 0) {
+          dbg0[alen] = left ? uint8_t('-') : uint8_t(s1[i - 1] & 15u);
+          dbg1[alen] = left ? uint8_t(s2[j - 1] & 15u) : uint8_t('-');
+        }
+        ++alen;
       }
-      ++alen;
-    }
+      j -= left;
+      i -= 1 - left;
+      t0 += 1 - left;
+      k += 1 - 2 * left;
+    } while (t0 < 32 && unsigned(k) < unsigned(N) && min(i, j) > 0);
   }
-  if (dbg0) {  // row 0 moves left, column 0 moves up
-    for (int t = lane; t < j; t += 32) { dbg0[alen + t] = '-'; dbg1[alen + t] = S.s2[j - 1 - t] & 15u; }
-    for (int t = lane; t < i; t += 32) { dbg0[alen + t] = S.s1[i - 1 - t] & 15u; dbg1[alen + t] = '-'; }
+  if (bad) {
+    if (lane == 0) atomicOr(err_word, DERR_TRACEBACK);
+    return false;
   }
-  alen += uint32_t(i + j);
+  if (DBG) {  // row 0 moves left, column 0 moves up
+    for (int t = lane; t < j; t += 32) { dbg0[alen + t] = '-'; dbg1[alen + t] = s2[j - 1 - t] & 15u; }
+    for (int t = lane; t < i; t += 32) { dbg0[alen + t] = s1[i - 1 - t] & 15u; dbg1[alen + t] = '-'; }
+    if (lane == 0) *dbg_len = alen + uint32_t(i + j);
+  }
   __syncwarp();
-  if (dbg_len && lane == 0) *dbg_len = alen;
-  *ham_out = ham;
+  *ham_out = __reduce_add_sync(FULL, mism);
   return true;
 }
 
@@ -154,7 +185,7 @@ __device__ __forceinline__ bool strip_traceback(int lane, int len1, int len2, in
 // add-max on the chain from its left neighbour.
 //
 // A cell's two pointer bits (diagonal best; else left better than up) are the
-// signs of differences, shifted into two words per lane: RPW = 32 / 2C rows
+// signs of differences, shifted into two words per lane: RPW = 16, 8, 4, 4 rows
 // per word, written as one 256-byte row of `planes` per RPW rows.
 //
 // The rows where some lane is before its first cell, or past the last row or
@@ -163,12 +194,12 @@ __device__ __forceinline__ bool strip_traceback(int lane, int len1, int len2, in
 // S.s1/S.s2 hold the codes, with the run flags when HOMO. Needs a band of
 // W <= 62 C diagonals, so that the lane after the last
 // one in use holds the mark outside the band (strip_cols).
-template <int C, bool HOMO>
-__device__ __noinline__ bool strip_align(int lane, int len1, int len2, int match, int mismatch, int gap, int hgap,
-                                         int band, const StripSmem& S, uint2* planes, bool in_smem,
+template <int C, bool HOMO, bool DBG>
+__device__ __forceinline__ bool strip_align(int lane, int len1, int len2, int match, int mismatch, int gap, int hgap,
+                                         int band, const StripSmem& S, uint2* planes,
                                          uint32_t* ham_out, uint32_t* err_word, uint8_t* dbg0, uint8_t* dbg1,
                                          uint32_t* dbg_len) {
-  constexpr int N = 2 * C, RPW = 32 / N;
+  constexpr int N = 2 * C, RPW = strip_rows_per_word(C);
   constexpr int BIG = 1 << 28;
   int o_lo, o_hi;
   band_offsets(band, len1, len2, &o_lo, &o_hi);
@@ -281,14 +312,14 @@ __device__ __noinline__ bool strip_align(int lane, int len1, int len2, int match
     *out = make_uint2(accD << sh, accL << sh);
   }
   __syncwarp();
-  return strip_traceback<C>(lane, len1, len2, o_lo, W, S, planes, in_smem, ham_out, err_word, dbg0, dbg1, dbg_len);
+  return strip_traceback<C, DBG>(lane, len1, len2, o_lo, W, S, planes, ham_out, err_word, dbg0, dbg1, dbg_len);
 }
 
 // The narrowest strip that holds the pair's band. CMAX bounds it for the
 // launch (the geometry's rule: strip_cols).
-template <int CMAX, bool HOMO>
+template <int CMAX, bool HOMO, bool DBG = false>
 __device__ __forceinline__ bool strip_dispatch(int lane, int len1, int len2, const KParams& kp, bool homo,
-                                               const StripSmem& S, uint2* planes, bool in_smem, uint32_t* ham,
+                                               const StripSmem& S, uint2* planes, uint32_t* ham,
                                                uint32_t* err_word, uint8_t* d0, uint8_t* d1, uint32_t* dl) {
   if (HOMO && homo) {
     flag_runs(lane, S.s1, len1);
@@ -301,7 +332,7 @@ __device__ __forceinline__ bool strip_dispatch(int lane, int len1, int len2, con
   const int need = strip_cols(o_hi - o_lo + 1);
 #define STRIP_CASE(CC)                                                                                            \
   if (CC == CMAX || need <= CC)                                                                                   \
-  return strip_align<CC, HOMO>(lane, len1, len2, kp.match, kp.mismatch, kp.gap, hg, kp.band, S, planes, in_smem, \
+  return strip_align<CC, HOMO, DBG>(lane, len1, len2, kp.match, kp.mismatch, kp.gap, hg, kp.band, S, planes, \
                                ham, err_word, d0, d1, dl)
   STRIP_CASE(1);
   if constexpr (CMAX >= 2) STRIP_CASE(2);
