@@ -73,7 +73,7 @@ struct TaskDev {
 // hdr); the offsets are from the header's own address.
 struct CallHeader {
   uint32_t ntask, total_items, screen_chunk, nstore_blocks;
-  uint32_t pivot, cdot_ready, total_cl, pad;
+  uint32_t pivot, cdot_ready, total_cl, direct;
   uint32_t o_tasks, o_pref, o_clp, o_map;
 };
 static_assert(sizeof(CallHeader) == 48, "the call header has a fixed layout");
@@ -84,7 +84,7 @@ enum : uint8_t { AM_NONE = 0, AM_GAPLESS = 1, AM_VECTORIZED = 2, AM_HOMO = 3, AM
 
 // Per-task counters written by the store kernel.
 enum { TC_SCREENED = 0, TC_ALIGNED, TC_SHROUD, TC_STORED, TC_GAPLESS, TC_VECTORIZED, TC_HOMO,
-       TC_ENDSFREE, TC_NCOUNTERS };
+       TC_ENDSFREE, TC_UNSET, TC_NCOUNTERS };  // TC_UNSET: raws whose e_minmax is still negative
 
 // Device error bits (OR-ed into the status word; the host turns them into codes).
 enum : uint32_t {
@@ -231,7 +231,8 @@ struct CompareLaunch {
   uint32_t total_cl;
   uint32_t* queue_pass;     // nraw capacity: items that passed the screen
   uint32_t* queue_counts;   // 8 words; [4] = items pushed to queue_pass, [5] = profiles the
-                            // screen read, [6] = the align warps' slot cursor
+                            // screen read, [6] = the align warps' slot cursor, [7] = blocks done
+                            // (direct store)
   uint8_t* nw_scratch;      // nwarps * nw_scratch_bytes(geom)
   NwGeom geom;
   uint32_t* err_word;
@@ -248,7 +249,16 @@ struct CompareLaunch {
   uint32_t* blk_counters;
   uint32_t nstore_blocks;
   int do_store;
-  // with do_store: the store's first CTA copies *err_word to err_host (mapped
+  // Direct store (with do_store, for calls whose tasks have no raw with a
+  // negative e_minmax): a raw that fails the screen has lambda 0 and can
+  // neither be stored nor move its e_minmax, so the screen only counts it, the
+  // alignment kernel stores each pair's comp itself, in any order, and its
+  // last block hands over the counters (task_ctr, ntask x TC_NCOUNTERS, zero
+  // between calls); there is no store kernel and blk_counters holds one row per
+  // task. At most kScreenSmemTasks tasks.
+  uint32_t direct;
+  uint32_t* task_ctr;
+  // with do_store: the store's first CTA (direct: the last align CTA) copies *err_word to err_host (mapped
   // host memory) and clears queue_counts for the launch context's next call
   uint32_t* err_host;
   // null: the fields above are this call's; else the launch is a graph

@@ -498,14 +498,16 @@ struct Slot {
   Pool* P = nullptr;
   cudaStream_t st = nullptr;
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
-  DBuf<uint32_t> queue_pass, queue_counts, err_dev;
+  DBuf<uint32_t> queue_pass, queue_counts, err_dev, task_ctr;
   DBuf<uint8_t> scratch;
   DBuf<uint8_t> dpack;  // tasks | task prefix | store map of the current launch
   HBuf<uint8_t> hpack;  // its pinned staging copy (one upload per launch)
   HBuf<uint32_t> blk_counters, err_host;
   HBuf<double> task_self;
   HBuf<TaskDev> task_stage;
-  std::vector<uint32_t> task_blk0;  // first store CTA of each task in the latest launch
+  std::vector<uint32_t> task_blk0;  // first store CTA (direct: the row) of each task in the latest launch
+  bool direct = false;              // the latest launch stored its comps directly
+  std::vector<std::vector<uint64_t>> order;  // then: each task's comps by raw, (index, place) packed
   uint32_t ntask_cap = 0, nblk_cap = 0;
   size_t pack_cap = 0;
   // Instantiated compare graphs, checked out of a per-device free list for
@@ -518,7 +520,7 @@ struct Slot {
   ~Slot() {
     if (st && cudaStreamSynchronize(st) == cudaSuccess && gs) graph_set_return(dev, gs);
     if (st && cudaStreamSynchronize(st) == cudaSuccess)  // every block is idle now
-      recycle_all(queue_pass, queue_counts, err_dev, scratch, dpack, hpack, blk_counters, err_host, task_self,
+      recycle_all(queue_pass, queue_counts, err_dev, task_ctr, scratch, dpack, hpack, blk_counters, err_host, task_self,
                   task_stage);
     for (auto& e : ev)
       if (e) cudaEventDestroy(e);
@@ -534,12 +536,14 @@ struct Slot {
     for (auto& e : ev) CUDA_TRY(cudaEventCreate(&e));
     TRY(queue_counts.alloc(8));
     TRY(err_dev.alloc(1));
+    TRY(task_ctr.alloc(size_t(kScreenSmemTasks) * TC_NCOUNTERS));
     TRY(err_host.alloc(2));  // [0] error flags, [1] profiles the screen read
     err_host.h[0] = 0;
     err_host.h[1] = 0;
     // both start at zero; every call leaves them at zero again
     CUDA_TRY(cudaMemsetAsync(queue_counts.p, 0, 32, st));
     CUDA_TRY(cudaMemsetAsync(err_dev.p, 0, 4, st));
+    CUDA_TRY(cudaMemsetAsync(task_ctr.p, 0, size_t(kScreenSmemTasks) * TC_NCOUNTERS * 4, st));
     CUDA_TRY(cudaStreamSynchronize(st));
     return 0;
   }
@@ -573,7 +577,9 @@ struct Slot {
   template <class F>
   void for_each_stored(uint32_t t, F&& f) const;
   void task_counters(uint32_t t, uint32_t* out) const;
-  int run_compare(uint32_t ntask, bool do_store, double* wait_s);
+  // may_direct: no raw of the tasks has a negative e_minmax, and few comps are
+  // expected (CompareLaunch::direct)
+  int run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_direct = false);
 };
 
 // Device pool: the resident uniques of one or more samples.
@@ -829,7 +835,13 @@ struct Pool {
 template <class F>
 void Slot::for_each_stored(uint32_t t, F&& f) const {
   const TaskDev& T = task_stage.h[t];
-  const uint32_t nb = (T.n + kStoreSpan - 1) / kStoreSpan;
+  const uint32_t nb = direct ? 0 : (T.n + kStoreSpan - 1) / kStoreSpan;
+  if (direct)
+    for (const uint64_t key : order[t]) {
+      const uint32_t o = T.out_off + uint32_t(key);
+      f(uint32_t(key >> 32), P->comp_lambda.h[o], P->comp_ham.h[o],
+        P->kp.lambda32 && P->comp_ll32.h ? P->comp_ll32.h[o] : std::numeric_limits<float>::quiet_NaN());
+    }
   for (uint32_t b = 0; b < nb; ++b) {
     const uint32_t cnt = blk_counters.h[size_t(task_blk0[t] + b) * TC_NCOUNTERS + TC_STORED];
     const uint32_t o = T.out_off + b * uint32_t(kStoreSpan);
@@ -843,24 +855,26 @@ void Slot::for_each_stored(uint32_t t, F&& f) const {
 // Counters of task t summed over its store CTAs.
 void Slot::task_counters(uint32_t t, uint32_t* out) const {
   for (int k = 0; k < TC_NCOUNTERS; ++k) out[k] = 0;
-  const uint32_t nb = (task_stage.h[t].n + kStoreSpan - 1) / kStoreSpan;
+  const uint32_t nb = direct ? 1 : (task_stage.h[t].n + kStoreSpan - 1) / kStoreSpan;
   for (uint32_t b = 0; b < nb; ++b)
     for (int k = 0; k < TC_NCOUNTERS; ++k) out[k] += blk_counters.h[size_t(task_blk0[t] + b) * TC_NCOUNTERS + k];
+  if (direct) out[TC_ALIGNED] = out[TC_GAPLESS] + out[TC_VECTORIZED] + out[TC_HOMO] + out[TC_ENDSFREE];
 }
 
 // Launches one compare over `ntask` tasks already in task_stage; waits for it.
 // The launch's tables go up in one copy; with the store, the error flags come
 // back through mapped memory and the queue counters are rearmed on the device.
-int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s) {
+int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_direct) {
   const auto t_call = Clock::now();
   TRY(ensure_tasks(ntask));
   const Pool& Q = *P;
+  direct = may_direct && do_store && Q.kp.use_kmers && ntask <= uint32_t(kScreenSmemTasks);
   uint32_t total = 0, nblk = 0;
   task_blk0.assign(ntask, 0);
   for (uint32_t t = 0; t < ntask; ++t) {
     task_stage.h[t].out_off = task_stage.h[t].base;
     task_blk0[t] = nblk;
-    nblk += (task_stage.h[t].n + kStoreSpan - 1) / kStoreSpan;
+    nblk += direct ? 1 : (task_stage.h[t].n + kStoreSpan - 1) / kStoreSpan;
   }
   TRY(ensure_blocks(nblk));
   // header | tasks | task prefix | cluster prefix | store map
@@ -876,7 +890,7 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s) {
   for (uint32_t t = 0; t < ntask; ++t) {
     pref[t] = total;
     total += task_stage.h[t].n;
-    const uint32_t nb = (task_stage.h[t].n + kStoreSpan - 1) / kStoreSpan;
+    const uint32_t nb = direct ? 1 : (task_stage.h[t].n + kStoreSpan - 1) / kStoreSpan;
     for (uint32_t b = 0; b < nb; ++b) {
       smap[task_blk0[t] + b] = t;
       smap[nblk + task_blk0[t] + b] = b;
@@ -906,6 +920,7 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s) {
     H.pivot = pivot ? 1u : 0u;
     H.cdot_ready = cdot_ready ? 1u : 0u;
     H.total_cl = cdot_ready ? total_cl : 0u;
+    H.direct = direct ? 1u : 0u;
     H.o_tasks = uint32_t(o_tasks);
     H.o_pref = uint32_t(o_pref);
     H.o_clp = uint32_t(o_clp);
@@ -936,6 +951,8 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s) {
   L.blk_counters = blk_counters.d;
   L.nstore_blocks = nblk;
   L.do_store = do_store ? 1 : 0;
+  L.direct = direct ? 1u : 0u;
+  L.task_ctr = task_ctr.p;
   L.err_host = err_host.d;
   {
     L.screen_chunk_max = uint32_t(tu.screen_chunk_max);
@@ -956,7 +973,7 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s) {
     // header just uploaded; the store grid is rounded up (spare CTAs return).
     CompareLaunch K = L;
     K.ntask = K.total_items = K.screen_chunk = K.nstore_blocks = 0;
-    K.pivot = K.cdot_ready = K.total_cl = 0;
+    K.pivot = K.cdot_ready = K.total_cl = K.direct = 0;
     K.tasks = nullptr;
     K.task_prefix = K.task_cl_prefix = K.store_task = K.store_chunk = nullptr;
     K.hdr = reinterpret_cast<const CallHeader*>(dpack.p);
@@ -971,8 +988,8 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s) {
     uint32_t sgrid = 64;
     while (sgrid < need && sgrid < wave) sgrid *= 2;
     sgrid = std::min(sgrid, wave);
-    uint32_t grid = 8;
-    while (grid < nblk) grid *= 4;
+    uint32_t grid = direct ? 0 : 8;  // 0: no store kernel
+    while (grid < nblk && !direct) grid *= 4;
     const uint32_t key = (sgrid << 20) ^ (grid << 1) ^ (cdot_ready ? 1u : 0u);
     GraphSet::Entry& E = gs->by_variant[key];
     if (!E.exec || std::memcmp(&E.key, &K, sizeof K) != 0) {
@@ -1031,7 +1048,7 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s) {
     dgpu_kernel_stats& S = g_stats.s;
     S.launches[1] += 1;
     S.launches[2] += 1;
-    if (do_store) S.launches[3] += 1;
+    if (do_store && !direct) S.launches[3] += 1;
     for (int k = 0; k < 3; ++k) S.ms[k + 1] += ms[k];
     S.rounds += 1;
     S.compares += total;
@@ -1067,6 +1084,15 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s) {
     CUDA_TRY(cudaMemsetAsync(err_dev.p, 0, 4, st));
     CUDA_TRY(cudaStreamSynchronize(st));
     return fail(ew & DERR_UNSUPPORTED ? DGPU_E_UNSUPPORTED : DGPU_E_DEVICE, "device error:" + what);
+  }
+  if (direct) {  // the comps in ascending raw order, as the store kernel gives them
+    if (order.size() < ntask) order.resize(ntask);
+    for (uint32_t t = 0; t < ntask; ++t) {
+      const uint32_t ns = blk_counters.h[size_t(t) * TC_NCOUNTERS + TC_STORED], o = task_stage.h[t].out_off;
+      order[t].resize(ns);
+      for (uint32_t k = 0; k < ns; ++k) order[t][k] = (uint64_t(Q.comp_index.h[o + k]) << 32) | k;
+      std::sort(order[t].begin(), order[t].end());
+    }
   }
   return 0;
 }
@@ -1303,6 +1329,10 @@ struct DadaConf {
   bool fp32 = false;  // decisions from the FP32 lambda, FP64 near the thresholds
 };
 
+// A call that may store this many comps takes the store kernel: ordering more
+// on the host costs what that kernel does (about 10 us).
+static constexpr uint32_t kDirectMax = 1024;
+
 struct SampleState {
   uint32_t n = 0, base = 0;
   uint32_t total_reads = 0;
@@ -1327,6 +1357,10 @@ struct SampleState {
   uint64_t nalign = 0, nshroud = 0;
   RunStats stats;
   bool lock_dirty = false, done = false;
+  // The next compare call may store directly: every raw's e_minmax is set, and
+  // the last call stored few comps (clusters come largest first, so the next
+  // stores about as few; the host orders a direct call's comps).
+  bool few_stored = false, e_set = false;
   int64_t pending = -1;  // cluster whose compare is queued
   // shuffle carry (src/cluster.rs:848-866)
   std::vector<Comp> compmax;
@@ -1568,6 +1602,9 @@ struct SampleState {
   template <class Each>
   void absorb_from(size_t ci, const uint32_t* ctr, double self, Each&& each) {
     const uint32_t ns = ctr[TC_STORED];
+    // a direct call's counters have TC_UNSET 0 and follow one that had
+    e_set = ctr[TC_UNSET] == 0;
+    few_stored = ns < kDirectMax;
     nalign += ctr[TC_SCREENED];
     nshroud += ctr[TC_SHROUD];
     stats.compare_calls++;
@@ -2946,10 +2983,12 @@ static int run_samples(Pool& P, std::vector<SampleState>& S, const dgpu_align_pa
           for (size_t sidx : batch) S[sidx].stats.t_slot_wait += secs(S[sidx].stats.t_mark, now);
         }
         int r = L.ensure_tasks(uint32_t(batch.size()));
+        bool direct = true;
         for (size_t a = 0; a < batch.size() && !r; ++a) {
           SampleState& ss = S[batch[a]];
           const size_t ci = size_t(ss.pending);
           L.task_stage.h[a] = ss.task_for(ci, ci == 0 ? 1.0 : ap.kdist_cutoff);  // init_params, src/dada.rs:835-838
+          direct = direct && ss.e_set && ss.few_stored;
           if (ss.lock_dirty) {
             r = P.push_locks(ss.base, ss.n, L.st);
             ss.lock_dirty = false;
@@ -2957,7 +2996,7 @@ static int run_samples(Pool& P, std::vector<SampleState>& S, const dgpu_align_pa
         }
         const auto tc = Clock::now();
         const double w0 = my_wait;
-        if (!r) r = L.run_compare(uint32_t(batch.size()), true, &my_wait);
+        if (!r) r = L.run_compare(uint32_t(batch.size()), true, &my_wait, direct);
         if (r) {
           std::lock_guard<std::mutex> g(mu);
           if (!rc) {
@@ -3366,7 +3405,7 @@ struct ShardHead {
   uint32_t has_self;  // the center lies in the rank's share
   uint32_t pad;
   double self;        // the center's own lambda, with has_self
-  uint32_t ctr[TC_NCOUNTERS];
+  uint32_t ctr[TC_UNSET];  // the call's counters (TC_UNSET is the rank's own affair)
 };
 struct ShardComp {
   uint32_t index, hamming;
@@ -3429,7 +3468,7 @@ static int shard_exchange(SampleState& S, size_t ci, const ShardHead& mine, cons
   uint32_t ctr[TC_NCOUNTERS] = {};
   double self = 0.0;
   for (const ShardHead& h : heads) {
-    for (int k = 0; k < TC_NCOUNTERS; ++k) ctr[k] += h.ctr[k];
+    for (int k = 0; k < TC_UNSET; ++k) ctr[k] += h.ctr[k];
     if (h.has_self) self = h.self;
   }
   S.absorb_from(ci, ctr, self, [&](auto&& f) {
@@ -3459,7 +3498,9 @@ static int shard_compare(Pool& P, SampleState& S, size_t ci, double cutoff, uint
   T.n = hi - lo;
   L.task_stage.h[0] = T;
   TRY(L.run_compare(1, true, nullptr));
-  L.task_counters(0, h.ctr);
+  uint32_t ctr[TC_NCOUNTERS];
+  L.task_counters(0, ctr);
+  std::copy(ctr, ctr + TC_UNSET, h.ctr);
   h.ns = h.ctr[TC_STORED];
   h.has_self = T.center >= T.base && T.center - T.base < T.n ? 1u : 0u;
   h.self = h.has_self ? L.task_self.h[0] : 0.0;

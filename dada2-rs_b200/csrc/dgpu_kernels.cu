@@ -295,6 +295,7 @@ __device__ __forceinline__ void load_call(CompareLaunch& L) {
   L.pivot = H.pivot;
   L.cdot_ready = H.cdot_ready;
   L.total_cl = H.total_cl;
+  L.direct = H.direct;
   L.tasks = reinterpret_cast<const TaskDev*>(base + H.o_tasks);
   L.task_prefix = reinterpret_cast<const uint32_t*>(base + H.o_pref);
   L.task_cl_prefix = reinterpret_cast<const uint32_t*>(base + H.o_clp);
@@ -359,6 +360,11 @@ __global__ void __launch_bounds__(kScreenWarps * 32, 4) k_screen(CompareLaunch L
   __shared__ uint32_t s_base[kScreenSmemTasks], s_center[kScreenSmemTasks], s_creads[kScreenSmemTasks];
   __shared__ double s_cutoff[kScreenSmemTasks];
   __shared__ uint32_t s_cluster[kScreenSmemTasks];
+  // direct store: this block's screened and shrouded raws per task
+  __shared__ uint32_t s_ctr[2 * kScreenSmemTasks];
+  const bool direct = L.direct != 0;
+  if (direct)
+    for (uint32_t t = threadIdx.x; t < 2 * L.ntask; t += blockDim.x) s_ctr[t] = 0;
   const bool tasks_smem = L.ntask <= uint32_t(kScreenSmemTasks);
   if (tasks_smem) {
     for (uint32_t t = threadIdx.x; t <= L.ntask; t += blockDim.x) {
@@ -578,33 +584,45 @@ __global__ void __launch_bounds__(kScreenWarps * 32, 4) k_screen(CompareLaunch L
       }
     }
     bool pass = false;
+    bool shroud = bounded;
     if (valid) {
-      if (kp.lambda32) L.pool.res_loglam32[g] = -INFINITY;
-      if (bounded) {
-        L.pool.res_lambda[g] = 0.0;
-        L.pool.res_ham[g] = 0xffffffffu;
-        L.pool.res_status[g] = ST_SHROUDED;
-      } else if (skip) {
-        L.pool.res_lambda[g] = 0.0;
-        L.pool.res_ham[g] = 0xffffffffu;
-        L.pool.res_status[g] = ST_SKIPPED;
-      } else {
+      if (kp.lambda32 && !direct) L.pool.res_loglam32[g] = -INFINITY;
+      if (!bounded && !skip) {
         double kdist = 0.0;
-        bool shroud = false;
         if (kp.use_kmers) {
           const int lc = int(L.pool.len[c]), lg = int(L.pool.len[g]);
           const int minl = lc < lg ? lc : lg;
           kdist = 1.0 - double(mydot) / double(minl - K + 1);
           shroud = kdist > (tasks_smem ? s_cutoff[t] : L.tasks[t].cutoff);
         }
-        if (shroud) {
-          L.pool.res_lambda[g] = 0.0;
-          L.pool.res_ham[g] = 0xffffffffu;
-          L.pool.res_status[g] = ST_SHROUDED;
-        } else {
+        if (!shroud) {
           L.pool.res_lambda[g] = kdist;
           pass = true;
         }
+      }
+      if (!pass) {
+        if (!direct) {
+          L.pool.res_lambda[g] = 0.0;
+          L.pool.res_ham[g] = 0xffffffffu;
+          L.pool.res_status[g] = shroud ? ST_SHROUDED : ST_SKIPPED;
+        } else if (g == c) {
+          L.task_self[t] = 0.0;
+        }
+      }
+    }
+    if (direct) {
+      // one task in most chunks: a ballot each; else every raw by itself
+      const uint32_t t0 = __shfl_sync(FULL, t, 0);  // a chunk's valid lanes are its first
+      const bool one = __all_sync(FULL, !valid || t == t0);
+      const uint32_t scr = __ballot_sync(FULL, valid && !skip), shr = __ballot_sync(FULL, valid && shroud);
+      if (one) {
+        if (lane == 0) {
+          atomicAdd(&s_ctr[2 * t], uint32_t(__popc(scr)));
+          atomicAdd(&s_ctr[2 * t + 1], uint32_t(__popc(shr)));
+        }
+      } else if (valid) {
+        if (!skip) atomicAdd(&s_ctr[2 * t], 1u);
+        if (shroud) atomicAdd(&s_ctr[2 * t + 1], 1u);
       }
     }
     const uint32_t pm = __ballot_sync(FULL, pass);
@@ -613,6 +631,13 @@ __global__ void __launch_bounds__(kScreenWarps * 32, 4) k_screen(CompareLaunch L
       if (lane == 0) base = atomicAdd(&L.queue_counts[4], uint32_t(__popc(pm)));
       base = __shfl_sync(FULL, base, 0);
       if (pass) L.queue_pass[base + __popc(pm & ((1u << lane) - 1u))] = item;
+    }
+  }
+  if (direct) {
+    __syncthreads();
+    for (uint32_t t = threadIdx.x; t < L.ntask; t += blockDim.x) {
+      if (s_ctr[2 * t]) atomicAdd(&L.task_ctr[t * TC_NCOUNTERS + TC_SCREENED], s_ctr[2 * t]);
+      if (s_ctr[2 * t + 1]) atomicAdd(&L.task_ctr[t * TC_NCOUNTERS + TC_SHROUD], s_ctr[2 * t + 1]);
     }
   }
 }
@@ -2534,7 +2559,8 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
   // or sixteen groups, G > 1 per warp) keep one warp per pair.
   constexpr bool STRIP = FORMS == kFormsStrip1 || FORMS == kFormsStrip;
   const bool coop = !STRIP && L.geom.vec_scratch == 0 && kb >= 2 && kb <= kNwWarps && count <= 2u * gridDim.x;
-  if (blockIdx.x >= count) return;  // nothing queued for this block
+  const bool direct = L.direct != 0;
+  if (blockIdx.x >= count && !direct) return;  // nothing queued for this block
   const size_t err_bytes = err_smem_bytes(kp.ncol);
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   // One warp of every block takes a short queue's pairs before any block uses
@@ -2546,8 +2572,9 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
   const size_t scr_stride = nw_scratch_bytes(L.geom);
   uint8_t* scratch = L.nw_scratch + size_t(gw) * scr_stride;
   __syncthreads();
-  // lambda and the raw's result entries, by the warp that holds the alignment
-  auto finish = [&](const PairResult& R, uint32_t g) {
+  // lambda and the raw's result entries (direct: its comp, if stored), by the
+  // warp that holds the alignment
+  auto finish = [&](const PairResult& R, uint32_t g, uint32_t t, const TaskDev& T) {
     double lam = 0.0;
     float ll32 = -INFINITY;
     if (R.ok) {
@@ -2560,13 +2587,50 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
         if (kp.lambda32) ll32 = loglambda32(lane, R.fidx, R.lg, err_s);
       }
     }
-    if (lane == 0) {
+    if (lane == 0 && direct) {
+      const double e = L.pool.e_minmax[g];
+      uint32_t* ctr = L.task_ctr + t * TC_NCOUNTERS;
+      if (__dmul_rn(lam, T.total_reads) > e) {  // k_store's rule (src/cluster.rs:379-396)
+        const double ne = __dmul_rn(lam, double(T.center_reads));
+        if (ne > e) L.pool.e_minmax[g] = ne;
+        const uint32_t o = T.out_off + atomicAdd(ctr + TC_STORED, 1u);
+        L.comp_index[o] = g - T.base;
+        L.comp_lambda[o] = lam;
+        L.comp_ham[o] = R.ok ? R.ham : 0u;
+        if (L.comp_ll32) L.comp_ll32[o] = ll32;
+      }
+      if (g == T.center) L.task_self[t] = lam;
+      if (R.method != AM_NONE) atomicAdd(ctr + TC_GAPLESS + R.method - AM_GAPLESS, 1u);
+    } else if (lane == 0) {
       if (kp.lambda32) L.pool.res_loglam32[g] = ll32;
       L.pool.res_lambda[g] = lam;
       L.pool.res_ham[g] = R.ok ? R.ham : 0xffffffffu;
       L.pool.res_status[g] = uint8_t(ST_ALIGNED | (R.method << 2));
     }
     __syncwarp();
+  };
+  // Direct store: the last block to finish hands the call's counters and error
+  // flags to the host and clears them for the next call, as k_store does.
+  auto close_call = [&] {
+    __shared__ uint32_t s_last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      s_last = atomicAdd(&L.queue_counts[7], 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    for (uint32_t k = threadIdx.x; k < L.ntask * TC_NCOUNTERS; k += blockDim.x) {
+      L.blk_counters[k] = *(volatile uint32_t*)&L.task_ctr[k];
+      L.task_ctr[k] = 0;
+    }
+    if (threadIdx.x == 0) {
+      reinterpret_cast<volatile uint32_t*>(L.err_host)[0] = *(volatile uint32_t*)L.err_word;
+      reinterpret_cast<volatile uint32_t*>(L.err_host)[1] = *(volatile uint32_t*)&L.queue_counts[5];
+    }
+    __syncthreads();
+    if (threadIdx.x < 8) L.queue_counts[threadIdx.x] = 0;
   };
   if constexpr (!STRIP) if (coop) {
     // Thread 0 claims a slot for the CTA and reads the raw's screen distance
@@ -2580,20 +2644,19 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
     const VecSmem VS0 = carve_vec(w0, L.geom.lmax, L.geom.vec_ncol);
     const RmSmem RS0 = carve_rm(w0, L.geom.lmax, kb);
     uint8_t* scratch0 = L.nw_scratch + size_t(blockIdx.x) * kNwWarps * scr_stride;
-    auto raw_of = [&](uint32_t slot, uint32_t* center) {
+    auto raw_of = [&](uint32_t slot, uint32_t* task) {
       const uint32_t item = L.queue_pass[slot];
       const uint32_t t = find_task(L.task_prefix, L.ntask, item);
-      const TaskDev T = L.tasks[t];
-      *center = T.center;
-      return T.base + (item - L.task_prefix[t]);
+      *task = t;
+      return L.tasks[t].base + (item - L.task_prefix[t]);
     };
     for (;;) {
       if (threadIdx.x == 0) {
         const uint32_t sl = atomicAdd(&L.queue_counts[6], 1u);
         s_slot = sl;
         if (sl < count) {
-          uint32_t c0;
-          s_kdist = L.pool.res_lambda[raw_of(sl, &c0)];
+          uint32_t t0;
+          s_kdist = L.pool.res_lambda[raw_of(sl, &t0)];
         }
       }
       __syncthreads();
@@ -2601,12 +2664,14 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
       const double kdist = slot < count ? s_kdist : 0.0;
       __syncthreads();  // every thread has read the slot before thread 0 claims again
       if (slot >= count) break;
-      uint32_t center;
-      const uint32_t g = raw_of(slot, &center);
-      const PairResult R = align_pair<true, FORMS>(lane, kp, L.pool, L.geom, g, center, kdist, kp.use_quals != 0, VS0, RS0,
+      uint32_t t;
+      const uint32_t g = raw_of(slot, &t);
+      const TaskDev T = L.tasks[t];
+      const PairResult R = align_pair<true, FORMS>(lane, kp, L.pool, L.geom, g, T.center, kdist, kp.use_quals != 0, VS0, RS0,
                                             kb, scratch0, L.err_word, wib, s_xch);
-      if (wib == 0) finish(R, g);
+      if (wib == 0) finish(R, g, t, T);
     }
+    if (direct) close_call();
     return;
   }
   // Warps claim queue slots one at a time from a shared cursor (cleared with
@@ -2614,9 +2679,8 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
   // against NW, short against long -- and CTAs that become resident late
   // (when shared memory admits fewer CTAs per SM than the grid assumes) even
   // out. Results go to each raw's own entries, so the order is free.
-  if (spare) return;
   auto each_pair = [&](auto&& align) {
-    for (;;) {
+    while (!spare) {
       uint32_t slot = 0;
       if (lane == 0) slot = atomicAdd(&L.queue_counts[6], 1u);
       slot = __shfl_sync(FULL, slot, 0);
@@ -2625,7 +2689,7 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
       const uint32_t t = find_task(L.task_prefix, L.ntask, item);
       const TaskDev T = L.tasks[t];
       const uint32_t g = T.base + (item - L.task_prefix[t]);
-      finish(align(g, T.center), g);
+      finish(align(g, T.center), g, t, T);
     }
   };
   if constexpr (STRIP) {
@@ -2642,6 +2706,7 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
                                       kb, scratch, L.err_word);
     });
   }
+  if (direct) close_call();
 }
 
 // ---------------------------------------------------------------------------
@@ -2762,7 +2827,7 @@ __global__ void __launch_bounds__(kStoreThreads) k_store(CompareLaunch Lp) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   if (threadIdx.x < TC_NCOUNTERS) ctr[threadIdx.x] = 0;
   __syncthreads();
-  uint32_t c_scr = 0, c_al = 0, c_sh = 0, c_gl = 0, c_ve = 0, c_ho = 0, c_ef = 0;
+  uint32_t c_scr = 0, c_al = 0, c_sh = 0, c_gl = 0, c_ve = 0, c_ho = 0, c_ef = 0, c_un = 0;
   const uint32_t r0 = span0 + threadIdx.x * IPT;
   uint32_t flags = 0;
   double lam[IPT];
@@ -2785,12 +2850,13 @@ __global__ void __launch_bounds__(kStoreThreads) k_store(CompareLaunch Lp) {
       c_ef += meth == AM_ENDSFREE;
       lam[q] = L.pool.res_lambda[g];
       ham[q] = L.pool.res_ham[g];
-      const double e = L.pool.e_minmax[g];
+      double e = L.pool.e_minmax[g];
       if (__dmul_rn(lam[q], T.total_reads) > e) {
         flags |= 1u << q;
         const double ne = __dmul_rn(lam[q], double(T.center_reads));
-        if (ne > e) L.pool.e_minmax[g] = ne;
+        if (ne > e) L.pool.e_minmax[g] = e = ne;
       }
+      c_un += !(e >= 0.0);
       if (g == T.center) L.task_self[t] = lam[q];
     }
   }
@@ -2848,6 +2914,7 @@ __global__ void __launch_bounds__(kStoreThreads) k_store(CompareLaunch Lp) {
   c_ve = __reduce_add_sync(FULL, c_ve);
   c_ho = __reduce_add_sync(FULL, c_ho);
   c_ef = __reduce_add_sync(FULL, c_ef);
+  c_un = __reduce_add_sync(FULL, c_un);
   if (lane == 0) {
     atomicAdd(&ctr[TC_SCREENED], c_scr);
     atomicAdd(&ctr[TC_ALIGNED], c_al);
@@ -2856,6 +2923,7 @@ __global__ void __launch_bounds__(kStoreThreads) k_store(CompareLaunch Lp) {
     atomicAdd(&ctr[TC_VECTORIZED], c_ve);
     atomicAdd(&ctr[TC_HOMO], c_ho);
     atomicAdd(&ctr[TC_ENDSFREE], c_ef);
+    atomicAdd(&ctr[TC_UNSET], c_un);
   }
   __syncthreads();
   if (threadIdx.x < TC_NCOUNTERS) L.blk_counters[size_t(blk) * TC_NCOUNTERS + threadIdx.x] = ctr[threadIdx.x];
@@ -3005,7 +3073,7 @@ void launch_compare(const CompareLaunch& L0, cudaStream_t st, cudaEvent_t* ev) {
                           ? std::min<uint32_t>((L.total_cl + 7) / 8, uint32_t(sms) * 8u)
                           : 0u;
   const size_t asm_ = err_smem_bytes(L.kp.ncol) + size_t(kNwWarps) * align_smem_per_warp(L.geom);
-  launch_chain(L, st, ev, blocks, pb, L.do_store ? L.nstore_blocks : 0u, align_kernel(L, asm_), asm_);
+  launch_chain(L, st, ev, blocks, pb, L.do_store && !L.direct ? L.nstore_blocks : 0u, align_kernel(L, asm_), asm_);
 }
 
 int capture_compare_graph(const CompareLaunch& L, cudaStream_t st, uint32_t screen_grid, bool pivot_dots,
