@@ -35,7 +35,7 @@ struct PoolDev {
   const uint8_t* kcnt;
   const uint32_t* knum;
   const uint32_t* reads;
-  const uint8_t* lock;
+  uint8_t* lock;
   double* e_minmax;
   const double* err;      // 16 x ncol
   // per-raw results of the latest compare launch
@@ -75,8 +75,9 @@ struct CallHeader {
   uint32_t ntask, total_items, screen_chunk, nstore_blocks;
   uint32_t pivot, cdot_ready, total_cl, direct;
   uint32_t o_tasks, o_pref, o_clp, o_map;
+  uint32_t nlock, o_lock;
 };
-static_assert(sizeof(CallHeader) == 48, "the call header has a fixed layout");
+static_assert(sizeof(CallHeader) == 56, "the call header has a fixed layout");
 
 // res_status layout: low 2 bits = outcome, next 3 bits = aligner.
 enum : uint8_t { ST_ALIGNED = 0, ST_SKIPPED = 1, ST_SHROUDED = 2 };
@@ -125,6 +126,7 @@ constexpr int kAlignCtasPerSm = 4; // resident align CTAs per SM (128 registers 
 constexpr int kStageBytes = 4096; // traceback staging per warp
 constexpr int kStripPad = 16;     // readable bytes past the strip aligner's staged sequences
 constexpr size_t kStripSmemMax = 8192;  // pointer words of a pair kept in shared memory up to this size
+constexpr uint32_t kLockListMax = 256;  // locks a direct call takes as a list
 constexpr uint32_t kNoPivot = 0xffffffffu;
 constexpr int kRmStageRows = 128; // anti-diagonals of pointer planes the row-major traceback stages at once
 constexpr int kStoreSpan = 2048;  // raws per store CTA (its own output segment)
@@ -255,9 +257,14 @@ struct CompareLaunch {
   // alignment kernel stores each pair's comp itself, in any order, and its
   // last block hands over the counters (task_ctr, ntask x TC_NCOUNTERS, zero
   // between calls); there is no store kernel and blk_counters holds one row per
-  // task. At most kScreenSmemTasks tasks.
+  // task. At most kScreenSmemTasks tasks. `direct` is the call's number (never
+  // 0), which the last block writes to err_host[2] when all else is done.
   uint32_t direct;
   uint32_t* task_ctr;
+  // direct: the raws locked since the tables' last call (at most kLockListMax);
+  // the screen enters them in pool.lock as it reads them
+  const uint32_t* lock_list;
+  uint32_t nlock;
   // with do_store: the store's first CTA (direct: the last align CTA) copies *err_word to err_host (mapped
   // host memory) and clears queue_counts for the launch context's next call
   uint32_t* err_host;

@@ -507,6 +507,8 @@ struct Slot {
   HBuf<TaskDev> task_stage;
   std::vector<uint32_t> task_blk0;  // first store CTA (direct: the row) of each task in the latest launch
   bool direct = false;              // the latest launch stored its comps directly
+  uint32_t direct_seq = 0;          // direct calls so far, never 0 in a call
+  std::vector<uint32_t> lock_list;  // raws locked since the last call, for a direct call's screen
   std::vector<std::vector<uint64_t>> order;  // then: each task's comps by raw, (index, place) packed
   uint32_t ntask_cap = 0, nblk_cap = 0;
   size_t pack_cap = 0;
@@ -537,9 +539,10 @@ struct Slot {
     TRY(queue_counts.alloc(8));
     TRY(err_dev.alloc(1));
     TRY(task_ctr.alloc(size_t(kScreenSmemTasks) * TC_NCOUNTERS));
-    TRY(err_host.alloc(2));  // [0] error flags, [1] profiles the screen read
+    TRY(err_host.alloc(3));  // [0] error flags, [1] profiles the screen read, [2] the last direct call done
     err_host.h[0] = 0;
     err_host.h[1] = 0;
+    err_host.h[2] = 0;
     // both start at zero; every call leaves them at zero again
     CUDA_TRY(cudaMemsetAsync(queue_counts.p, 0, 32, st));
     CUDA_TRY(cudaMemsetAsync(err_dev.p, 0, 4, st));
@@ -577,7 +580,9 @@ struct Slot {
   template <class F>
   void for_each_stored(uint32_t t, F&& f) const;
   void task_counters(uint32_t t, uint32_t* out) const;
-  // may_direct: no raw of the tasks has a negative e_minmax, and few comps are
+  // whether a call of ntask tasks can store directly
+  bool direct_fits(uint32_t ntask) const;
+  // may_direct: direct_fits, no raw of the tasks has a negative e_minmax, and few comps are
   // expected (CompareLaunch::direct)
   int run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_direct = false);
 };
@@ -831,6 +836,10 @@ struct Pool {
   }
 };
 
+bool Slot::direct_fits(uint32_t ntask) const {
+  return P->kp.use_kmers && ntask <= uint32_t(kScreenSmemTasks);
+}
+
 // Stored comps of task t (latest launch), in ascending raw order.
 template <class F>
 void Slot::for_each_stored(uint32_t t, F&& f) const {
@@ -868,7 +877,7 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_di
   const auto t_call = Clock::now();
   TRY(ensure_tasks(ntask));
   const Pool& Q = *P;
-  direct = may_direct && do_store && Q.kp.use_kmers && ntask <= uint32_t(kScreenSmemTasks);
+  direct = may_direct && do_store;
   uint32_t total = 0, nblk = 0;
   task_blk0.assign(ntask, 0);
   for (uint32_t t = 0; t < ntask; ++t) {
@@ -882,9 +891,13 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_di
   const size_t o_pref = o_tasks + align16(sizeof(TaskDev) * ntask);
   const size_t o_clp = o_pref + align16(size_t(4) * (ntask + 1));
   const size_t o_map = o_clp + align16(size_t(4) * (ntask + 1));
-  const size_t pack_bytes = o_map + align16(size_t(8) * std::max<uint32_t>(nblk, 1));
+  const size_t o_lock = o_map + align16(size_t(8) * std::max<uint32_t>(nblk, 1));
+  const uint32_t nlock = direct ? uint32_t(lock_list.size()) : 0u;
+  const size_t pack_bytes = o_lock + align16(size_t(4) * std::max<uint32_t>(nlock, 1));
+  if (direct && ++direct_seq == 0) direct_seq = 1;
   TRY(ensure_pack(pack_bytes));
   std::memcpy(hpack.h + o_tasks, task_stage.h, sizeof(TaskDev) * ntask);
+  if (nlock) std::memcpy(hpack.h + o_lock, lock_list.data(), size_t(4) * nlock);
   uint32_t* pref = reinterpret_cast<uint32_t*>(hpack.h + o_pref);
   uint32_t* smap = reinterpret_cast<uint32_t*>(hpack.h + o_map);
   for (uint32_t t = 0; t < ntask; ++t) {
@@ -920,7 +933,9 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_di
     H.pivot = pivot ? 1u : 0u;
     H.cdot_ready = cdot_ready ? 1u : 0u;
     H.total_cl = cdot_ready ? total_cl : 0u;
-    H.direct = direct ? 1u : 0u;
+    H.direct = direct ? direct_seq : 0u;
+    H.nlock = nlock;
+    H.o_lock = uint32_t(o_lock);
     H.o_tasks = uint32_t(o_tasks);
     H.o_pref = uint32_t(o_pref);
     H.o_clp = uint32_t(o_clp);
@@ -951,7 +966,9 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_di
   L.blk_counters = blk_counters.d;
   L.nstore_blocks = nblk;
   L.do_store = do_store ? 1 : 0;
-  L.direct = direct ? 1u : 0u;
+  L.direct = direct ? direct_seq : 0u;
+  L.lock_list = reinterpret_cast<const uint32_t*>(dpack.p + o_lock);
+  L.nlock = nlock;
   L.task_ctr = task_ctr.p;
   L.err_host = err_host.d;
   {
@@ -973,7 +990,8 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_di
     // header just uploaded; the store grid is rounded up (spare CTAs return).
     CompareLaunch K = L;
     K.ntask = K.total_items = K.screen_chunk = K.nstore_blocks = 0;
-    K.pivot = K.cdot_ready = K.total_cl = K.direct = 0;
+    K.pivot = K.cdot_ready = K.total_cl = K.direct = K.nlock = 0;
+    K.lock_list = nullptr;
     K.tasks = nullptr;
     K.task_prefix = K.task_cl_prefix = K.store_task = K.store_chunk = nullptr;
     K.hdr = reinterpret_cast<const CallHeader*>(dpack.p);
@@ -1030,7 +1048,18 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_di
   // Poll and yield rather than block in the driver's spin: the launch slots'
   // threads share the cores with the host phases they wait for (on B200 with
   // 16 host cores the 40-sample step went from 79-82 ms to 75-78 ms).
-  const cudaError_t q = poll_with_limit([&] { return cudaStreamQuery(st); }, wait_limit_s());
+  // A direct call's last block reports in mapped memory, 3 to 6 us before the
+  // stream does; the stream is asked now and then for an error.
+  uint32_t polls = 0;
+  auto query = [&]() -> cudaError_t {
+    if (!direct || timing) return cudaStreamQuery(st);
+    if (*static_cast<volatile uint32_t*>(err_host.h + 2) == direct_seq) {
+      std::atomic_thread_fence(std::memory_order_acquire);
+      return cudaSuccess;
+    }
+    return ++polls % 256 ? cudaErrorNotReady : cudaStreamQuery(st);
+  };
+  const cudaError_t q = poll_with_limit(query, wait_limit_s());
   if (q == cudaErrorTimeout)
     return fail(DGPU_E_CUDA, "compare launch still running after the wait limit (DGPU_WAIT_LIMIT_S, default 300 s); "
                              "the context must not be reused");
@@ -1361,6 +1390,7 @@ struct SampleState {
   // the last call stored few comps (clusters come largest first, so the next
   // stores about as few; the host orders a direct call's comps).
   bool few_stored = false, e_set = false;
+  std::vector<uint32_t> lock_new;  // raws locked since the last call, up to one past kLockListMax
   int64_t pending = -1;  // cluster whose compare is queued
   // shuffle carry (src/cluster.rs:848-866)
   std::vector<Comp> compmax;
@@ -1975,6 +2005,7 @@ struct SampleState {
           if (l && !lock[raw]) {
             lock[raw] = 1;
             lock_dirty = true;
+            if (lock_new.size() <= kLockListMax) lock_new.push_back(base + raw);
           }
         }
         bi.check_locks = false;
@@ -2983,16 +3014,25 @@ static int run_samples(Pool& P, std::vector<SampleState>& S, const dgpu_align_pa
           for (size_t sidx : batch) S[sidx].stats.t_slot_wait += secs(S[sidx].stats.t_mark, now);
         }
         int r = L.ensure_tasks(uint32_t(batch.size()));
-        bool direct = true;
+        bool direct = L.direct_fits(uint32_t(batch.size()));
         for (size_t a = 0; a < batch.size() && !r; ++a) {
           SampleState& ss = S[batch[a]];
           const size_t ci = size_t(ss.pending);
           L.task_stage.h[a] = ss.task_for(ci, ci == 0 ? 1.0 : ap.kdist_cutoff);  // init_params, src/dada.rs:835-838
           direct = direct && ss.e_set && ss.few_stored;
-          if (ss.lock_dirty) {
+        }
+        // locks set since a sample's last call: the direct call's screen enters
+        // a short list of them itself; else the sample's flags are copied
+        L.lock_list.clear();
+        for (size_t a = 0; a < batch.size() && !r; ++a) {
+          SampleState& ss = S[batch[a]];
+          if (!ss.lock_dirty) continue;
+          if (direct && L.lock_list.size() + ss.lock_new.size() <= kLockListMax)
+            L.lock_list.insert(L.lock_list.end(), ss.lock_new.begin(), ss.lock_new.end());
+          else
             r = P.push_locks(ss.base, ss.n, L.st);
-            ss.lock_dirty = false;
-          }
+          ss.lock_dirty = false;
+          ss.lock_new.clear();
         }
         const auto tc = Clock::now();
         const double w0 = my_wait;
@@ -3490,6 +3530,7 @@ static int shard_compare(Pool& P, SampleState& S, size_t ci, double cutoff, uint
   if (S.lock_dirty) {
     TRY(P.push_locks(S.base, S.n, L.st));
     S.lock_dirty = false;
+    S.lock_new.clear();
   }
   if (lo == hi) return 0;
   TRY(L.ensure_tasks(1));

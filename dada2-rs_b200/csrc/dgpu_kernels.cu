@@ -296,6 +296,8 @@ __device__ __forceinline__ void load_call(CompareLaunch& L) {
   L.cdot_ready = H.cdot_ready;
   L.total_cl = H.total_cl;
   L.direct = H.direct;
+  L.nlock = H.nlock;
+  L.lock_list = reinterpret_cast<const uint32_t*>(base + H.o_lock);
   L.tasks = reinterpret_cast<const TaskDev*>(base + H.o_tasks);
   L.task_prefix = reinterpret_cast<const uint32_t*>(base + H.o_pref);
   L.task_cl_prefix = reinterpret_cast<const uint32_t*>(base + H.o_clp);
@@ -363,8 +365,13 @@ __global__ void __launch_bounds__(kScreenWarps * 32, 4) k_screen(CompareLaunch L
   // direct store: this block's screened and shrouded raws per task
   __shared__ uint32_t s_ctr[2 * kScreenSmemTasks];
   const bool direct = L.direct != 0;
-  if (direct)
+  __shared__ uint4 s_lock[kLockListMax / 4];
+  const uint32_t nlock4 = direct ? (L.nlock + 3) / 4 : 0u;
+  if (direct) {
     for (uint32_t t = threadIdx.x; t < 2 * L.ntask; t += blockDim.x) s_ctr[t] = 0;
+    for (uint32_t t = threadIdx.x; t < 4 * nlock4; t += blockDim.x)
+      reinterpret_cast<uint32_t*>(s_lock)[t] = t < L.nlock ? L.lock_list[t] : 0xffffffffu;
+  }
   const bool tasks_smem = L.ntask <= uint32_t(kScreenSmemTasks);
   if (tasks_smem) {
     for (uint32_t t = threadIdx.x; t <= L.ntask; t += blockDim.x) {
@@ -413,7 +420,15 @@ __global__ void __launch_bounds__(kScreenWarps * 32, 4) k_screen(CompareLaunch L
       const uint32_t tn = (tasks_smem ? s_prefix[t + 1] : L.task_prefix[t + 1]) - t0;
       g = tbase + (item - t0);
       cl_fits = ccl < tn;  // cluster indices of a whole sample stay below its raw count
-      skip = kp.greedy && (L.pool.reads[g] > creads || L.pool.lock[g]);
+      bool locked = L.pool.lock[g] != 0;
+      if (!locked && nlock4) {
+        for (uint32_t q = 0; q < nlock4; ++q) {
+          const uint4 x = s_lock[q];
+          locked |= x.x == g || x.y == g || x.z == g || x.w == g;
+        }
+        if (locked) L.pool.lock[g] = 1;
+      }
+      skip = kp.greedy && (L.pool.reads[g] > creads || locked);
       if (pivot && !skip) {
         // Exact exclusion without reading the raw's profile. For non-negative
         // count vectors min(c, r) <= min(c, p) + r - min(r, p) elementwise, so
@@ -2571,6 +2586,8 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
   unsigned char* wbase = smem_raw + err_bytes + size_t(wib) * align_smem_per_warp(L.geom);
   const size_t scr_stride = nw_scratch_bytes(L.geom);
   uint8_t* scratch = L.nw_scratch + size_t(gw) * scr_stride;
+  __shared__ uint32_t s_host;  // direct: the block wrote to host memory
+  if (threadIdx.x == 0) s_host = 0;
   __syncthreads();
   // lambda and the raw's result entries (direct: its comp, if stored), by the
   // warp that holds the alignment
@@ -2593,13 +2610,17 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
       if (__dmul_rn(lam, T.total_reads) > e) {  // k_store's rule (src/cluster.rs:379-396)
         const double ne = __dmul_rn(lam, double(T.center_reads));
         if (ne > e) L.pool.e_minmax[g] = ne;
+        s_host = 1;
         const uint32_t o = T.out_off + atomicAdd(ctr + TC_STORED, 1u);
         L.comp_index[o] = g - T.base;
         L.comp_lambda[o] = lam;
         L.comp_ham[o] = R.ok ? R.ham : 0u;
         if (L.comp_ll32) L.comp_ll32[o] = ll32;
       }
-      if (g == T.center) L.task_self[t] = lam;
+      if (g == T.center) {
+        s_host = 1;
+        L.task_self[t] = lam;
+      }
       if (R.method != AM_NONE) atomicAdd(ctr + TC_GAPLESS + R.method - AM_GAPLESS, 1u);
     } else if (lane == 0) {
       if (kp.lambda32) L.pool.res_loglam32[g] = ll32;
@@ -2615,7 +2636,8 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
     __shared__ uint32_t s_last;
     __syncthreads();
     if (threadIdx.x == 0) {
-      __threadfence();
+      if (s_host) __threadfence_system();
+      else __threadfence();
       s_last = atomicAdd(&L.queue_counts[7], 1u) == gridDim.x - 1;
     }
     __syncthreads();
@@ -2631,6 +2653,9 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
     }
     __syncthreads();
     if (threadIdx.x < 8) L.queue_counts[threadIdx.x] = 0;
+    __threadfence_system();
+    __syncthreads();
+    if (threadIdx.x == 0) reinterpret_cast<volatile uint32_t*>(L.err_host)[2] = L.direct;
   };
   if constexpr (!STRIP) if (coop) {
     // Thread 0 claims a slot for the CTA and reads the raw's screen distance
