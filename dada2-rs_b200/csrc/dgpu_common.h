@@ -127,6 +127,10 @@ constexpr int kStageBytes = 4096; // traceback staging per warp
 constexpr int kStripPad = 16;     // readable bytes past the strip aligner's staged sequences
 constexpr size_t kStripSmemMax = 8192;  // pointer words of a pair kept in shared memory up to this size
 constexpr uint32_t kLockListMax = 256;  // locks a direct call takes as a list
+constexpr uint32_t kPostHead = 2 + 2 * kScreenSmemTasks;  // units before a direct call's pairs
+constexpr uint32_t kPostMax = 4096;       // pairs a direct call posts
+// bits of a posted pair: mismatches, aligner, stored, device error, task
+constexpr uint32_t kPostMethod = 14, kPostStored = 17, kPostError = 18, kPostTask = 19;
 constexpr uint32_t kNoPivot = 0xffffffffu;
 constexpr int kRmStageRows = 128; // anti-diagonals of pointer planes the row-major traceback stages at once
 constexpr int kStoreSpan = 2048;  // raws per store CTA (its own output segment)
@@ -253,19 +257,27 @@ struct CompareLaunch {
   int do_store;
   // Direct store (with do_store, for calls whose tasks have no raw with a
   // negative e_minmax): a raw that fails the screen has lambda 0 and can
-  // neither be stored nor move its e_minmax, so the screen only counts it, the
-  // alignment kernel stores each pair's comp itself, in any order, and its
-  // last block hands over the counters (task_ctr, ntask x TC_NCOUNTERS, zero
-  // between calls); there is no store kernel and blk_counters holds one row per
-  // task. At most kScreenSmemTasks tasks. `direct` is the call's number (never
-  // 0), which the last block writes to err_host[2] when all else is done.
+  // neither be stored nor move its e_minmax, so the screen only counts it, each
+  // aligned pair is stored and posted to the host by its own warp, and there is
+  // no store kernel. At most kScreenSmemTasks tasks, without lambda32. `direct`
+  // is the call's number (never 0) and task_ctr, ntask x 2, the screened and
+  // shrouded raws (zero between calls).
+  //
+  // Posts are 8-byte units in mapped host memory, the value in the low half and
+  // the call's number in the high half, so each says by itself that it is
+  // there and nothing waits for a fence: unit 0 the pairs queued, unit 1 the
+  // profiles read, then two units per task from task_ctr; from unit kPostHead
+  // on four units per pair, by queue slot: the raw, kPost* bits, lambda's
+  // halves. A call that queues more than kPostMax pairs posts its head only
+  // and aligns none: the host makes the call again with the store kernel.
   uint32_t direct;
   uint32_t* task_ctr;
+  uint64_t* post;
   // direct: the raws locked since the tables' last call (at most kLockListMax);
   // the screen enters them in pool.lock as it reads them
   const uint32_t* lock_list;
   uint32_t nlock;
-  // with do_store: the store's first CTA (direct: the last align CTA) copies *err_word to err_host (mapped
+  // with do_store: the store's first CTA (direct: the last align CTA, after the posts) copies *err_word to err_host (mapped
   // host memory) and clears queue_counts for the launch context's next call
   uint32_t* err_host;
   // null: the fields above are this call's; else the launch is a graph

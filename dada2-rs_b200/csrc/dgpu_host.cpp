@@ -509,7 +509,12 @@ struct Slot {
   bool direct = false;              // the latest launch stored its comps directly
   uint32_t direct_seq = 0;          // direct calls so far, never 0 in a call
   std::vector<uint32_t> lock_list;  // raws locked since the last call, for a direct call's screen
-  std::vector<std::vector<uint64_t>> order;  // then: each task's comps by raw, (index, place) packed
+  // then: each task's counters, and its stored comps in ascending raw order as
+  // (raw index, queue slot) packed
+  std::vector<std::array<uint32_t, TC_NCOUNTERS>> dctr;
+  std::vector<std::vector<uint64_t>> order;
+  HBuf<uint64_t> post;  // its posts (CompareLaunch::post)
+  uint32_t posted = 0, post_err = 0;  // units read so far, and whether a pair told of an error
   uint32_t ntask_cap = 0, nblk_cap = 0;
   size_t pack_cap = 0;
   // Instantiated compare graphs, checked out of a per-device free list for
@@ -523,7 +528,7 @@ struct Slot {
     if (st && cudaStreamSynchronize(st) == cudaSuccess && gs) graph_set_return(dev, gs);
     if (st && cudaStreamSynchronize(st) == cudaSuccess)  // every block is idle now
       recycle_all(queue_pass, queue_counts, err_dev, task_ctr, scratch, dpack, hpack, blk_counters, err_host, task_self,
-                  task_stage);
+                  task_stage, post);
     for (auto& e : ev)
       if (e) cudaEventDestroy(e);
     if (st) cudaStreamDestroy(st);
@@ -538,15 +543,16 @@ struct Slot {
     for (auto& e : ev) CUDA_TRY(cudaEventCreate(&e));
     TRY(queue_counts.alloc(8));
     TRY(err_dev.alloc(1));
-    TRY(task_ctr.alloc(size_t(kScreenSmemTasks) * TC_NCOUNTERS));
-    TRY(err_host.alloc(3));  // [0] error flags, [1] profiles the screen read, [2] the last direct call done
+    TRY(task_ctr.alloc(size_t(kScreenSmemTasks) * 2));
+    TRY(post.alloc(kPostHead + size_t(4) * kPostMax));
+    std::memset(post.h, 0, (kPostHead + size_t(4) * kPostMax) * 8);  // no call has number 0
+    TRY(err_host.alloc(2));  // [0] error flags, [1] profiles the screen read
     err_host.h[0] = 0;
     err_host.h[1] = 0;
-    err_host.h[2] = 0;
     // both start at zero; every call leaves them at zero again
     CUDA_TRY(cudaMemsetAsync(queue_counts.p, 0, 32, st));
     CUDA_TRY(cudaMemsetAsync(err_dev.p, 0, 4, st));
-    CUDA_TRY(cudaMemsetAsync(task_ctr.p, 0, size_t(kScreenSmemTasks) * TC_NCOUNTERS * 4, st));
+    CUDA_TRY(cudaMemsetAsync(task_ctr.p, 0, size_t(kScreenSmemTasks) * 2 * 4, st));
     CUDA_TRY(cudaStreamSynchronize(st));
     return 0;
   }
@@ -585,6 +591,11 @@ struct Slot {
   // may_direct: direct_fits, no raw of the tasks has a negative e_minmax, and few comps are
   // expected (CompareLaunch::direct)
   int run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_direct = false);
+  // whether every post of the latest direct call has come
+  bool posts_here(uint32_t ntask);
+  // the call's counters and comps from its posts; false: it queued more pairs
+  // than it posts and has to be made again with the store kernel
+  bool read_posts(uint32_t ntask);
 };
 
 // Device pool: the resident uniques of one or more samples.
@@ -836,8 +847,14 @@ struct Pool {
   }
 };
 
+static double f64_of(uint64_t bits) {
+  double d;
+  std::memcpy(&d, &bits, sizeof d);
+  return d;
+}
+
 bool Slot::direct_fits(uint32_t ntask) const {
-  return P->kp.use_kmers && ntask <= uint32_t(kScreenSmemTasks);
+  return P->kp.use_kmers && !P->kp.lambda32 && ntask <= uint32_t(kScreenSmemTasks);
 }
 
 // Stored comps of task t (latest launch), in ascending raw order.
@@ -847,9 +864,10 @@ void Slot::for_each_stored(uint32_t t, F&& f) const {
   const uint32_t nb = direct ? 0 : (T.n + kStoreSpan - 1) / kStoreSpan;
   if (direct)
     for (const uint64_t key : order[t]) {
-      const uint32_t o = T.out_off + uint32_t(key);
-      f(uint32_t(key >> 32), P->comp_lambda.h[o], P->comp_ham.h[o],
-        P->kp.lambda32 && P->comp_ll32.h ? P->comp_ll32.h[o] : std::numeric_limits<float>::quiet_NaN());
+      const uint64_t* u = post.h + kPostHead + 4 * uint32_t(key);
+      const uint64_t lam = (u[3] << 32) | (u[2] & 0xffffffffu);
+      f(uint32_t(key >> 32), f64_of(lam), uint32_t(u[1]) & ((1u << kPostMethod) - 1),
+        std::numeric_limits<float>::quiet_NaN());
     }
   for (uint32_t b = 0; b < nb; ++b) {
     const uint32_t cnt = blk_counters.h[size_t(task_blk0[t] + b) * TC_NCOUNTERS + TC_STORED];
@@ -863,11 +881,58 @@ void Slot::for_each_stored(uint32_t t, F&& f) const {
 
 // Counters of task t summed over its store CTAs.
 void Slot::task_counters(uint32_t t, uint32_t* out) const {
-  for (int k = 0; k < TC_NCOUNTERS; ++k) out[k] = 0;
-  const uint32_t nb = direct ? 1 : (task_stage.h[t].n + kStoreSpan - 1) / kStoreSpan;
+  for (int k = 0; k < TC_NCOUNTERS; ++k) out[k] = direct ? dctr[t][k] : 0;
+  const uint32_t nb = direct ? 0 : (task_stage.h[t].n + kStoreSpan - 1) / kStoreSpan;
   for (uint32_t b = 0; b < nb; ++b)
     for (int k = 0; k < TC_NCOUNTERS; ++k) out[k] += blk_counters.h[size_t(task_blk0[t] + b) * TC_NCOUNTERS + k];
-  if (direct) out[TC_ALIGNED] = out[TC_GAPLESS] + out[TC_VECTORIZED] + out[TC_HOMO] + out[TC_ENDSFREE];
+}
+
+bool Slot::posts_here(uint32_t ntask) {
+  const volatile uint64_t* u = post.h;
+  const uint32_t head = 2 + 2 * ntask;
+  auto here = [&](uint32_t k) { return uint32_t(u[k] >> 32) == direct_seq; };
+  while (posted < head) {
+    if (!here(posted)) return false;
+    ++posted;
+  }
+  const uint32_t queued = uint32_t(u[0]), npair = queued > kPostMax ? 0 : queued;
+  for (; posted < head + 4 * npair; ++posted) {
+    const uint32_t k = kPostHead + posted - head;
+    if (!here(k)) return false;
+    if ((posted - head) % 4 == 1) post_err |= uint32_t(u[k]) & (1u << kPostError);
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  return true;
+}
+
+bool Slot::read_posts(uint32_t ntask) {
+  const uint64_t* u = post.h;
+  const uint32_t queued = uint32_t(u[0]);
+  err_host.h[1] = uint32_t(u[1]);
+  if (queued > kPostMax) return false;
+  if (order.size() < ntask) order.resize(ntask);
+  if (dctr.size() < ntask) dctr.resize(ntask);
+  for (uint32_t t = 0; t < ntask; ++t) {
+    order[t].clear();
+    dctr[t].fill(0);
+    dctr[t][TC_SCREENED] = uint32_t(u[2 + 2 * t]);
+    dctr[t][TC_SHROUD] = uint32_t(u[3 + 2 * t]);
+    task_self.h[t] = 0.0;  // unless the center's own pair says otherwise
+  }
+  for (uint32_t q = 0; q < queued; ++q) {
+    const uint64_t* e = u + kPostHead + 4 * q;
+    const uint32_t g = uint32_t(e[0]), bits = uint32_t(e[1]), t = bits >> kPostTask;
+    const TaskDev& T = task_stage.h[t];
+    dctr[t][TC_ALIGNED] += 1;
+    dctr[t][TC_GAPLESS - AM_GAPLESS + ((bits >> kPostMethod) & 7u)] += 1;
+    if (g == T.center) task_self.h[t] = f64_of((e[3] << 32) | (e[2] & 0xffffffffu));
+    if (bits & (1u << kPostStored)) order[t].push_back((uint64_t(g - T.base) << 32) | q);
+  }
+  for (uint32_t t = 0; t < ntask; ++t) {
+    dctr[t][TC_STORED] = uint32_t(order[t].size());
+    std::sort(order[t].begin(), order[t].end());
+  }
+  return true;
 }
 
 // Launches one compare over `ntask` tasks already in task_stage; waits for it.
@@ -883,7 +948,7 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_di
   for (uint32_t t = 0; t < ntask; ++t) {
     task_stage.h[t].out_off = task_stage.h[t].base;
     task_blk0[t] = nblk;
-    nblk += direct ? 1 : (task_stage.h[t].n + kStoreSpan - 1) / kStoreSpan;
+    nblk += direct ? 0 : (task_stage.h[t].n + kStoreSpan - 1) / kStoreSpan;
   }
   TRY(ensure_blocks(nblk));
   // header | tasks | task prefix | cluster prefix | store map
@@ -895,6 +960,7 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_di
   const uint32_t nlock = direct ? uint32_t(lock_list.size()) : 0u;
   const size_t pack_bytes = o_lock + align16(size_t(4) * std::max<uint32_t>(nlock, 1));
   if (direct && ++direct_seq == 0) direct_seq = 1;
+  posted = post_err = 0;
   TRY(ensure_pack(pack_bytes));
   std::memcpy(hpack.h + o_tasks, task_stage.h, sizeof(TaskDev) * ntask);
   if (nlock) std::memcpy(hpack.h + o_lock, lock_list.data(), size_t(4) * nlock);
@@ -903,7 +969,7 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_di
   for (uint32_t t = 0; t < ntask; ++t) {
     pref[t] = total;
     total += task_stage.h[t].n;
-    const uint32_t nb = direct ? 1 : (task_stage.h[t].n + kStoreSpan - 1) / kStoreSpan;
+    const uint32_t nb = direct ? 0 : (task_stage.h[t].n + kStoreSpan - 1) / kStoreSpan;
     for (uint32_t b = 0; b < nb; ++b) {
       smap[task_blk0[t] + b] = t;
       smap[nblk + task_blk0[t] + b] = b;
@@ -970,6 +1036,7 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_di
   L.lock_list = reinterpret_cast<const uint32_t*>(dpack.p + o_lock);
   L.nlock = nlock;
   L.task_ctr = task_ctr.p;
+  L.post = post.d;
   L.err_host = err_host.d;
   {
     L.screen_chunk_max = uint32_t(tu.screen_chunk_max);
@@ -1048,18 +1115,18 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_di
   // Poll and yield rather than block in the driver's spin: the launch slots'
   // threads share the cores with the host phases they wait for (on B200 with
   // 16 host cores the 40-sample step went from 79-82 ms to 75-78 ms).
-  // A direct call's last block reports in mapped memory, 3 to 6 us before the
-  // stream does; the stream is asked now and then for an error.
+  // A direct call's posts come some 10 us before the stream is done; the
+  // stream is asked now and then for an error.
   uint32_t polls = 0;
   auto query = [&]() -> cudaError_t {
     if (!direct || timing) return cudaStreamQuery(st);
-    if (*static_cast<volatile uint32_t*>(err_host.h + 2) == direct_seq) {
-      std::atomic_thread_fence(std::memory_order_acquire);
-      return cudaSuccess;
-    }
+    if (posts_here(ntask)) return cudaSuccess;
     return ++polls % 256 ? cudaErrorNotReady : cudaStreamQuery(st);
   };
-  const cudaError_t q = poll_with_limit(query, wait_limit_s());
+  cudaError_t q = poll_with_limit(query, wait_limit_s());
+  // a pair that failed: the flags come when the kernel is done
+  if (direct && q == cudaSuccess && (timing || !posts_here(ntask) || post_err))
+    q = poll_with_limit([&] { return cudaStreamQuery(st); }, wait_limit_s());
   if (q == cudaErrorTimeout)
     return fail(DGPU_E_CUDA, "compare launch still running after the wait limit (DGPU_WAIT_LIMIT_S, default 300 s); "
                              "the context must not be reused");
@@ -1071,7 +1138,9 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_di
     if (timing)
       for (int k = 0; k < 3; ++k) CUDA_TRY(cudaEventElapsedTime(&ms[k], ev[k], ev[k + 1]));
     uint64_t screened = 0;
-    if (do_store)
+    if (direct && posts_here(ntask))
+      for (uint32_t t = 0; t < ntask; ++t) screened += uint32_t(post.h[2 + 2 * t]);
+    else if (do_store && !direct)
       for (uint32_t b = 0; b < nblk; ++b) screened += blk_counters.h[size_t(b) * TC_NCOUNTERS + TC_SCREENED];
     std::lock_guard<std::mutex> g(g_stats.mu);
     dgpu_kernel_stats& S = g_stats.s;
@@ -1089,7 +1158,7 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_di
     // pivot when the loop keeps pivots; and both profiles of each center dot
     const uint64_t prof = Q.kp.kmer_size >= 8 ? uint64_t(3) * (Q.lmax - uint32_t(Q.kp.kmer_size) + 1)
                                               : (uint64_t(1) << (2 * Q.kp.kmer_size));
-    const uint64_t nread = Q.kp.kmer_size >= 8 ? screened : uint64_t(err_host.h[1]);
+    const uint64_t nread = Q.kp.kmer_size >= 8 ? screened : direct ? uint64_t(uint32_t(post.h[1])) : uint64_t(err_host.h[1]);
     const uint64_t sb = nread * prof + uint64_t(total) * (pivot ? 24u : 16u) +
                         (cdot_ready ? uint64_t(total_cl) * 2u * prof : 0u);
     S.screen_bytes += sb;
@@ -1114,15 +1183,9 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_di
     CUDA_TRY(cudaStreamSynchronize(st));
     return fail(ew & DERR_UNSUPPORTED ? DGPU_E_UNSUPPORTED : DGPU_E_DEVICE, "device error:" + what);
   }
-  if (direct) {  // the comps in ascending raw order, as the store kernel gives them
-    if (order.size() < ntask) order.resize(ntask);
-    for (uint32_t t = 0; t < ntask; ++t) {
-      const uint32_t ns = blk_counters.h[size_t(t) * TC_NCOUNTERS + TC_STORED], o = task_stage.h[t].out_off;
-      order[t].resize(ns);
-      for (uint32_t k = 0; k < ns; ++k) order[t][k] = (uint64_t(Q.comp_index.h[o + k]) << 32) | k;
-      std::sort(order[t].begin(), order[t].end());
-    }
-  }
+  if (direct && !posts_here(ntask)) return fail(DGPU_E_DEVICE, "device error: a compare call ended without its posts");
+  // too many pairs for a direct call, none of which it aligned
+  if (direct && !read_posts(ntask)) return run_compare(ntask, do_store, wait_s, false);
   return 0;
 }
 
@@ -1358,10 +1421,6 @@ struct DadaConf {
   bool fp32 = false;  // decisions from the FP32 lambda, FP64 near the thresholds
 };
 
-// A call that may store this many comps takes the store kernel: ordering more
-// on the host costs what that kernel does (about 10 us).
-static constexpr uint32_t kDirectMax = 1024;
-
 struct SampleState {
   uint32_t n = 0, base = 0;
   uint32_t total_reads = 0;
@@ -1387,9 +1446,9 @@ struct SampleState {
   RunStats stats;
   bool lock_dirty = false, done = false;
   // The next compare call may store directly: every raw's e_minmax is set, and
-  // the last call stored few comps (clusters come largest first, so the next
-  // stores about as few; the host orders a direct call's comps).
-  bool few_stored = false, e_set = false;
+  // the last call aligned few pairs (clusters come largest first, so the next
+  // aligns about as few; more than kPostMax would make the call twice).
+  bool few_pairs = false, e_set = false;
   std::vector<uint32_t> lock_new;  // raws locked since the last call, up to one past kLockListMax
   int64_t pending = -1;  // cluster whose compare is queued
   // shuffle carry (src/cluster.rs:848-866)
@@ -1634,7 +1693,7 @@ struct SampleState {
     const uint32_t ns = ctr[TC_STORED];
     // a direct call's counters have TC_UNSET 0 and follow one that had
     e_set = ctr[TC_UNSET] == 0;
-    few_stored = ns < kDirectMax;
+    few_pairs = ctr[TC_ALIGNED] < kPostMax / 4;
     nalign += ctr[TC_SCREENED];
     nshroud += ctr[TC_SHROUD];
     stats.compare_calls++;
@@ -3019,7 +3078,7 @@ static int run_samples(Pool& P, std::vector<SampleState>& S, const dgpu_align_pa
           SampleState& ss = S[batch[a]];
           const size_t ci = size_t(ss.pending);
           L.task_stage.h[a] = ss.task_for(ci, ci == 0 ? 1.0 : ap.kdist_cutoff);  // init_params, src/dada.rs:835-838
-          direct = direct && ss.e_set && ss.few_stored;
+          direct = direct && ss.e_set && ss.few_pairs;
         }
         // locks set since a sample's last call: the direct call's screen enters
         // a short list of them itself; else the sample's flags are copied

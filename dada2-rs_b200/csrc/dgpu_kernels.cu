@@ -313,6 +313,7 @@ template <int K>
 __global__ void __launch_bounds__(256) k_pivot_dots(CompareLaunch Lp) {
   CompareLaunch L = Lp;
   load_call(L);
+  cudaTriggerProgrammaticLaunchCompletion();  // the screen may start launching
   if (!L.cdot_ready) return;
   constexpr int NK16 = (1 << (2 * K)) / 16;
   const int lane = threadIdx.x & 31;
@@ -395,6 +396,8 @@ __global__ void __launch_bounds__(kScreenWarps * 32, 4) k_screen(CompareLaunch L
       const TaskDev T = L.tasks[t];
       if (T.cluster < T.n) L.pool.cl_center[T.base + T.cluster] = T.center;
     }
+  // launched as a dependent of k_pivot_dots, whose dots the bound reads
+  if (pivot && L.cdot_ready) cudaGridDependencySynchronize();
   const uint32_t CH = L.screen_chunk;  // lanes [0, CH) carry an item
   for (uint32_t chunk = (blockIdx.x * kScreenWarps + wib) * CH; chunk < L.total_items; chunk += warps_total * CH) {
     const uint32_t item = chunk + lane;
@@ -615,14 +618,10 @@ __global__ void __launch_bounds__(kScreenWarps * 32, 4) k_screen(CompareLaunch L
           pass = true;
         }
       }
-      if (!pass) {
-        if (!direct) {
-          L.pool.res_lambda[g] = 0.0;
-          L.pool.res_ham[g] = 0xffffffffu;
-          L.pool.res_status[g] = shroud ? ST_SHROUDED : ST_SKIPPED;
-        } else if (g == c) {
-          L.task_self[t] = 0.0;
-        }
+      if (!pass && !direct) {
+        L.pool.res_lambda[g] = 0.0;
+        L.pool.res_ham[g] = 0xffffffffu;
+        L.pool.res_status[g] = shroud ? ST_SHROUDED : ST_SKIPPED;
       }
     }
     if (direct) {
@@ -651,8 +650,8 @@ __global__ void __launch_bounds__(kScreenWarps * 32, 4) k_screen(CompareLaunch L
   if (direct) {
     __syncthreads();
     for (uint32_t t = threadIdx.x; t < L.ntask; t += blockDim.x) {
-      if (s_ctr[2 * t]) atomicAdd(&L.task_ctr[t * TC_NCOUNTERS + TC_SCREENED], s_ctr[2 * t]);
-      if (s_ctr[2 * t + 1]) atomicAdd(&L.task_ctr[t * TC_NCOUNTERS + TC_SHROUD], s_ctr[2 * t + 1]);
+      if (s_ctr[2 * t]) atomicAdd(&L.task_ctr[2 * t], s_ctr[2 * t]);
+      if (s_ctr[2 * t + 1]) atomicAdd(&L.task_ctr[2 * t + 1], s_ctr[2 * t + 1]);
     }
   }
 }
@@ -2566,7 +2565,9 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
   const int nerr = 16 * kp.ncol;
   for (int t = threadIdx.x; t < nerr; t += blockDim.x) err_s[t] = L.pool.err[t];
   cudaGridDependencySynchronize();  // the screen's pass queue and results are complete
-  const uint32_t count = *(volatile uint32_t*)&L.queue_counts[4];
+  const uint32_t queued = *(volatile uint32_t*)&L.queue_counts[4];
+  // a direct call with more pairs than its posts hold aligns none
+  const uint32_t count = L.direct && queued > kPostMax ? 0u : queued;
   const int kb = rm_kbound(L.geom.rm_pairs);
   // Few pairs of a launch whose NW pairs are all row-major and span two to
   // four lane groups: the CTA's warps share each pair (rm_align_coop), which
@@ -2578,26 +2579,28 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
   if (blockIdx.x >= count && !direct) return;  // nothing queued for this block
   const size_t err_bytes = err_smem_bytes(kp.ncol);
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  // One warp of every block takes a short queue's pairs before any block uses
-  // a second, so that the pairs spread over the SMs instead of filling the
-  // first blocks (a call with about 740 pairs of 1,450 nt: 0.77 -> 0.43 ms).
-  const bool spare = uint32_t(wib) * gridDim.x + blockIdx.x >= count;
   const int gw = blockIdx.x * kNwWarps + wib;
   unsigned char* wbase = smem_raw + err_bytes + size_t(wib) * align_smem_per_warp(L.geom);
   const size_t scr_stride = nw_scratch_bytes(L.geom);
   uint8_t* scratch = L.nw_scratch + size_t(gw) * scr_stride;
-  __shared__ uint32_t s_host;  // direct: the block wrote to host memory
-  if (threadIdx.x == 0) s_host = 0;
+  auto post = [&](uint32_t unit, uint32_t v) {
+    *reinterpret_cast<volatile uint64_t*>(L.post + unit) = (uint64_t(L.direct) << 32) | v;
+  };
+  if (direct && blockIdx.x == 0)
+    for (uint32_t u = threadIdx.x; u < 2 + 2 * L.ntask; u += blockDim.x)
+      post(u, u == 0 ? queued : *(volatile uint32_t*)(u == 1 ? &L.queue_counts[5] : &L.task_ctr[u - 2]));
   __syncthreads();
-  // lambda and the raw's result entries (direct: its comp, if stored), by the
-  // warp that holds the alignment
-  auto finish = [&](const PairResult& R, uint32_t g, uint32_t t, const TaskDev& T) {
+  // lambda and the raw's result entries (direct: its comp, if stored, and the
+  // pair's post), by the warp that holds the alignment; e: the raw's e_minmax
+  auto finish = [&](const PairResult& R, uint32_t g, uint32_t t, const TaskDev& T, uint32_t slot, double e) {
     double lam = 0.0;
+    bool failed = !R.ok;
     float ll32 = -INFINITY;
     if (R.ok) {
       const bool bad = build_fidx(lane, R.tcode, R.qual, R.lg, kp.ncol, kp.use_quals, R.fidx);
       __syncwarp();
       if (bad) {
+        failed = true;
         if (lane == 0) atomicOr(L.err_word, DERR_LAMBDA);
       } else {
         lam = lambda_chain(lane, R.fidx, R.lg, err_s);
@@ -2605,23 +2608,18 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
       }
     }
     if (lane == 0 && direct) {
-      const double e = L.pool.e_minmax[g];
-      uint32_t* ctr = L.task_ctr + t * TC_NCOUNTERS;
-      if (__dmul_rn(lam, T.total_reads) > e) {  // k_store's rule (src/cluster.rs:379-396)
+      const bool stored = __dmul_rn(lam, T.total_reads) > e;  // k_store's rule (src/cluster.rs:379-396)
+      if (stored) {
         const double ne = __dmul_rn(lam, double(T.center_reads));
         if (ne > e) L.pool.e_minmax[g] = ne;
-        s_host = 1;
-        const uint32_t o = T.out_off + atomicAdd(ctr + TC_STORED, 1u);
-        L.comp_index[o] = g - T.base;
-        L.comp_lambda[o] = lam;
-        L.comp_ham[o] = R.ok ? R.ham : 0u;
-        if (L.comp_ll32) L.comp_ll32[o] = ll32;
       }
-      if (g == T.center) {
-        s_host = 1;
-        L.task_self[t] = lam;
-      }
-      if (R.method != AM_NONE) atomicAdd(ctr + TC_GAPLESS + R.method - AM_GAPLESS, 1u);
+      const uint32_t bits = R.ham | (uint32_t(R.method) << kPostMethod) | (uint32_t(stored) << kPostStored) |
+                            (uint32_t(failed) << kPostError) | (t << kPostTask);
+      const uint32_t u = kPostHead + 4 * slot;
+      post(u, g);
+      post(u + 1, failed ? 1u << kPostError : bits);
+      post(u + 2, uint32_t(__double2loint(lam)));
+      post(u + 3, uint32_t(__double2hiint(lam)));
     } else if (lane == 0) {
       if (kp.lambda32) L.pool.res_loglam32[g] = ll32;
       L.pool.res_lambda[g] = lam;
@@ -2630,32 +2628,22 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
     }
     __syncwarp();
   };
-  // Direct store: the last block to finish hands the call's counters and error
-  // flags to the host and clears them for the next call, as k_store does.
+  // Direct store: the last block to finish clears the counters for the next
+  // call and hands over the error flags, which the host reads when a pair's
+  // post tells of one.
   auto close_call = [&] {
     __shared__ uint32_t s_last;
     __syncthreads();
     if (threadIdx.x == 0) {
-      if (s_host) __threadfence_system();
-      else __threadfence();
+      __threadfence();
       s_last = atomicAdd(&L.queue_counts[7], 1u) == gridDim.x - 1;
     }
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    for (uint32_t k = threadIdx.x; k < L.ntask * TC_NCOUNTERS; k += blockDim.x) {
-      L.blk_counters[k] = *(volatile uint32_t*)&L.task_ctr[k];
-      L.task_ctr[k] = 0;
-    }
-    if (threadIdx.x == 0) {
-      reinterpret_cast<volatile uint32_t*>(L.err_host)[0] = *(volatile uint32_t*)L.err_word;
-      reinterpret_cast<volatile uint32_t*>(L.err_host)[1] = *(volatile uint32_t*)&L.queue_counts[5];
-    }
-    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < 2 * L.ntask; k += blockDim.x) L.task_ctr[k] = 0;
+    if (threadIdx.x == 0) reinterpret_cast<volatile uint32_t*>(L.err_host)[0] = *(volatile uint32_t*)L.err_word;
     if (threadIdx.x < 8) L.queue_counts[threadIdx.x] = 0;
-    __threadfence_system();
-    __syncthreads();
-    if (threadIdx.x == 0) reinterpret_cast<volatile uint32_t*>(L.err_host)[2] = L.direct;
   };
   if constexpr (!STRIP) if (coop) {
     // Thread 0 claims a slot for the CTA and reads the raw's screen distance
@@ -2694,27 +2682,30 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
       const TaskDev T = L.tasks[t];
       const PairResult R = align_pair<true, FORMS>(lane, kp, L.pool, L.geom, g, T.center, kdist, kp.use_quals != 0, VS0, RS0,
                                             kb, scratch0, L.err_word, wib, s_xch);
-      if (wib == 0) finish(R, g, t, T);
+      if (wib == 0) finish(R, g, t, T, slot, L.pool.e_minmax[g]);
     }
     if (direct) close_call();
     return;
   }
-  // Warps claim queue slots one at a time from a shared cursor (cleared with
-  // the other counters after each call), so pairs of unequal cost -- gapless
+  // One warp of every block takes a short queue's pairs before any block uses
+  // a second, so that the pairs spread over the SMs instead of filling the
+  // first blocks (a call with about 740 pairs of 1,450 nt: 0.77 -> 0.43 ms).
+  // After that warps claim queue slots one at a time from a shared cursor
+  // (cleared with the other counters after each call), so pairs of unequal cost -- gapless
   // against NW, short against long -- and CTAs that become resident late
   // (when shared memory admits fewer CTAs per SM than the grid assumes) even
   // out. Results go to each raw's own entries, so the order is free.
   auto each_pair = [&](auto&& align) {
-    while (!spare) {
-      uint32_t slot = 0;
-      if (lane == 0) slot = atomicAdd(&L.queue_counts[6], 1u);
-      slot = __shfl_sync(FULL, slot, 0);
-      if (slot >= count) break;
+    // the first slot is the warp's own, the rest come from the cursor
+    for (uint32_t slot = uint32_t(wib) * gridDim.x + blockIdx.x; slot < count;) {
       const uint32_t item = L.queue_pass[slot];
       const uint32_t t = find_task(L.task_prefix, L.ntask, item);
       const TaskDev T = L.tasks[t];
       const uint32_t g = T.base + (item - L.task_prefix[t]);
-      finish(align(g, T.center), g, t, T);
+      const double e = direct ? L.pool.e_minmax[g] : 0.0;
+      finish(align(g, T.center), g, t, T, slot, e);
+      if (lane == 0) slot = kNwWarps * gridDim.x + atomicAdd(&L.queue_counts[6], 1u);
+      slot = __shfl_sync(FULL, slot, 0);
     }
   };
   if constexpr (STRIP) {
@@ -3050,24 +3041,28 @@ static void launch_chain(const CompareLaunch& L, cudaStream_t st, cudaEvent_t* e
       default: k_pivot_dots<7><<<pivot_blocks, 256, 0, st>>>(L); break;
     }
   }
-  switch (L.kp.kmer_size) {
-    case 3: k_screen<3><<<screen_blocks, kScreenWarps * 32, 0, st>>>(L); break;
-    case 4: k_screen<4><<<screen_blocks, kScreenWarps * 32, 0, st>>>(L); break;
-    case 5: k_screen<5><<<screen_blocks, kScreenWarps * 32, 0, st>>>(L); break;
-    case 6: k_screen<6><<<screen_blocks, kScreenWarps * 32, 0, st>>>(L); break;
-    case 7: k_screen<7><<<screen_blocks, kScreenWarps * 32, 0, st>>>(L); break;
-    default: k_screen<8><<<screen_blocks, kScreenWarps * 32, 0, st>>>(L); break;
-  }
-  if (ev) cudaEventRecord(ev[1], st);
-  // Programmatic dependent launch: the alignment and store kernels are
-  // scheduled while their predecessor drains and wait for its results in
-  // cudaGridDependencySynchronize, so the launch gaps overlap with work.
+  // Programmatic dependent launch: the alignment and store kernels, and the
+  // screen after k_pivot_dots, are scheduled while their predecessor drains and
+  // wait for its results in cudaGridDependencySynchronize, so the launch gaps
+  // overlap with work (the screen started 3.4 us after the dots' end before).
   cudaLaunchAttribute pdl[1];
   pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   pdl[0].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.stream = st;
   cfg.attrs = pdl;
+  cfg.numAttrs = L.pdl && pivot_blocks > 0 ? 1 : 0;
+  cfg.gridDim = dim3(screen_blocks);
+  cfg.blockDim = dim3(kScreenWarps * 32);
+  switch (L.kp.kmer_size) {
+    case 3: cudaLaunchKernelEx(&cfg, k_screen<3>, L); break;
+    case 4: cudaLaunchKernelEx(&cfg, k_screen<4>, L); break;
+    case 5: cudaLaunchKernelEx(&cfg, k_screen<5>, L); break;
+    case 6: cudaLaunchKernelEx(&cfg, k_screen<6>, L); break;
+    case 7: cudaLaunchKernelEx(&cfg, k_screen<7>, L); break;
+    default: cudaLaunchKernelEx(&cfg, k_screen<8>, L); break;
+  }
+  if (ev) cudaEventRecord(ev[1], st);
   cfg.numAttrs = L.pdl ? 1 : 0;
   cfg.gridDim = dim3(L.geom.nwarps / kNwWarps);
   cfg.blockDim = dim3(kNwWarps * 32);
