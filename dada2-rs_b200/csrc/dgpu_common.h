@@ -277,6 +277,7 @@ struct CompareLaunch {
   // the screen enters them in pool.lock as it reads them
   const uint32_t* lock_list;
   uint32_t nlock;
+  // (without do_store: k_collect writes the flags, the profiles read and the pairs queued)
   // with do_store: the store's first CTA (direct: the last align CTA, after the posts) copies *err_word to err_host (mapped
   // host memory) and clears queue_counts for the launch context's next call
   uint32_t* err_host;

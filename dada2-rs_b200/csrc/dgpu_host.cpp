@@ -546,9 +546,10 @@ struct Slot {
     TRY(task_ctr.alloc(size_t(kScreenSmemTasks) * 2));
     TRY(post.alloc(kPostHead + size_t(4) * kPostMax));
     std::memset(post.h, 0, (kPostHead + size_t(4) * kPostMax) * 8);  // no call has number 0
-    TRY(err_host.alloc(2));  // [0] error flags, [1] profiles the screen read
+    TRY(err_host.alloc(3));  // [0] error flags, [1] profiles the screen read, [2] pairs queued (without a store)
     err_host.h[0] = 0;
     err_host.h[1] = 0;
+    err_host.h[2] = 0;
     // both start at zero; every call leaves them at zero again
     CUDA_TRY(cudaMemsetAsync(queue_counts.p, 0, 32, st));
     CUDA_TRY(cudaMemsetAsync(err_dev.p, 0, 4, st));
@@ -1106,11 +1107,6 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_di
   }
   if (!launched) launch_compare(L, st, timing ? ev : nullptr);
   CUDA_TRY(cudaGetLastError());
-  if (!do_store) {  // no store kernel to rearm the queue or report the flags
-    CUDA_TRY(cudaMemcpyAsync(err_host.h, err_dev.p, 4, cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaMemcpyAsync(err_host.h + 1, queue_counts.p + 5, 4, cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaMemsetAsync(queue_counts.p, 0, 32, st));
-  }
   auto t0 = Clock::now();
   // Poll and yield rather than block in the driver's spin: the launch slots'
   // threads share the cores with the host phases they wait for (on B200 with
@@ -3670,6 +3666,7 @@ struct dgpu_ctx {
   dgpu::KParams kp{};
   std::vector<double> err;
   std::vector<uint32_t> reads;
+  uint64_t total_reads = 0;
   bool uploaded = false;
 };
 
@@ -3764,6 +3761,8 @@ int dgpu_upload_raws(dgpu_ctx* ctx, int nraw, const uint8_t* seqs, const uint32_
         if (quals[offs[t] + p] >= ctx->kp.ncol) return fail(DGPU_E_INVALID, "quality beyond the error matrix");
   }
   ctx->reads.assign(reads, reads + nraw);
+  ctx->total_reads = 0;
+  for (uint32_t r : ctx->reads) ctx->total_reads += r;
   TRY(ctx->pool.upload(uint32_t(nraw), seqs, offs, lens, quals, reads, ctx->kp, ctx->err.data()));
   ctx->uploaded = true;
   return 0;
@@ -3798,9 +3797,7 @@ static int ctx_task(dgpu_ctx* ctx, int center, int cluster_i, double cutoff, int
   T.n = ctx->pool.nraw;
   T.center = uint32_t(center);
   T.center_reads = ctx->reads[size_t(center)];
-  uint64_t tot = 0;
-  for (uint32_t r : ctx->reads) tot += r;
-  T.total_reads = double(uint32_t(tot));
+  T.total_reads = double(uint32_t(ctx->total_reads));
   T.cutoff = cutoff;
   T.cluster = uint32_t(cluster_i);
   ctx->pool.slot0().task_stage.h[0] = T;
@@ -3841,26 +3838,52 @@ int dgpu_compare(dgpu_ctx* ctx, int center, double kdist_cutoff, int greedy, dou
                  uint32_t* hamming_out, uint8_t* skipped_out, dgpu_counters* cnt) {
   TRY(ctx_task(ctx, center, 0, kdist_cutoff, greedy));
   Pool& P = ctx->pool;
-  TRY(P.slot0().run_compare(1, false, nullptr));
+  // Every raw's outcome before the pairs: skipped by the greedy rule on the
+  // host's own reads and locks (src/cluster.rs:295-298), else shrouded. The
+  // output pages are mostly new to the process and their faults cost a large
+  // call more than the device does, so a few threads fill them meanwhile.
   const uint32_t n = P.nraw;
-  std::vector<uint8_t> st(n);
-  if (lambda_out) CUDA_TRY(cudaMemcpy(lambda_out, P.lambda.p, size_t(n) * 8, cudaMemcpyDeviceToHost));
-  if (hamming_out) CUDA_TRY(cudaMemcpy(hamming_out, P.ham.p, size_t(n) * 4, cudaMemcpyDeviceToHost));
-  CUDA_TRY(cudaMemcpy(st.data(), P.status.p, n, cudaMemcpyDeviceToHost));
-  if (skipped_out)
-    for (uint32_t t = 0; t < n; ++t) skipped_out[t] = (st[t] & 3u) == ST_SKIPPED;
-  if (cnt) {
-    uint32_t c[TC_NCOUNTERS] = {0};
-    for (uint32_t t = 0; t < n; ++t) {
-      const uint8_t o = st[t] & 3u, m = st[t] >> 2;
-      c[TC_SCREENED] += o != ST_SKIPPED;
-      c[TC_ALIGNED] += o == ST_ALIGNED;
-      c[TC_SHROUD] += o == ST_SHROUDED;
-      c[TC_GAPLESS] += m == AM_GAPLESS;
-      c[TC_VECTORIZED] += m == AM_VECTORIZED;
-      c[TC_HOMO] += m == AM_HOMO;
-      c[TC_ENDSFREE] += m == AM_ENDSFREE;
+  const uint32_t creads = ctx->reads[size_t(center)];
+  const uint8_t* lock = P.lock_host.h;
+  std::atomic<uint64_t> nskip{0};
+  auto fill = [&](uint32_t lo, uint32_t hi) {
+    if (lambda_out) std::fill(lambda_out + lo, lambda_out + hi, 0.0);
+    if (hamming_out) std::fill(hamming_out + lo, hamming_out + hi, UINT32_MAX);
+    if (skipped_out && !greedy) std::fill(skipped_out + lo, skipped_out + hi, uint8_t(0));
+    uint64_t skips = 0;
+    for (uint32_t t = lo; greedy && t < hi; ++t) {
+      const uint8_t s = (ctx->reads[t] > creads) | (lock[t] != 0);
+      skips += s;
+      if (skipped_out) skipped_out[t] = s;
     }
+    nskip += skips;
+  };
+  std::thread filler;
+  if (n >= 65536)
+    filler = std::thread([&] {
+      const uint32_t parts = std::min(6u, std::max(1u, std::thread::hardware_concurrency() / 2));
+      auto part = [&](uint32_t k) { fill(uint32_t(uint64_t(n) * k / parts), uint32_t(uint64_t(n) * (k + 1) / parts)); };
+      std::vector<std::thread> th;
+      for (uint32_t k = 1; k < parts; ++k) th.emplace_back(part, k);
+      part(0);
+      for (auto& t : th) t.join();
+    });
+  const int rc = P.slot0().run_compare(1, false, nullptr);
+  if (filler.joinable()) filler.join();
+  else if (!rc) fill(0, n);
+  if (rc) return rc;
+  const uint32_t queued = P.slot0().err_host.h[2];
+  uint32_t c[TC_NCOUNTERS] = {0};
+  for (uint32_t q = 0; q < queued; ++q) {
+    const uint32_t g = P.comp_index.h[q], bits = P.comp_ham.h[q];
+    if (lambda_out) lambda_out[g] = P.comp_lambda.h[q];
+    if (hamming_out) hamming_out[g] = bits & ((1u << kPostMethod) - 1);
+    c[TC_GAPLESS - AM_GAPLESS + (bits >> kPostMethod)] += 1;
+  }
+  if (cnt) {
+    c[TC_SCREENED] = n - uint32_t(nskip.load());
+    c[TC_ALIGNED] = queued;
+    c[TC_SHROUD] = c[TC_SCREENED] - queued;
     fill_counters(c, 0, cnt);
   }
   return 0;

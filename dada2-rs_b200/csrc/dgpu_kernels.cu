@@ -2955,6 +2955,39 @@ __global__ void __launch_bounds__(kStoreThreads) k_store(CompareLaunch Lp) {
   }
 }
 
+// Without a store the host gets the aligned pairs alone, by queue slot, in the
+// comp arrays (comp_ham with the aligner above kPostMethod); every other raw's
+// outcome follows from the host's own reads and locks. A call over 400,000
+// uniques moves 0.4 MB for its 28,000 pairs, not the 5.2 MB of every raw's
+// entries. Its first block rearms the queue, as k_store's does.
+__global__ void __launch_bounds__(256) k_collect(CompareLaunch L) {
+  cudaGridDependencySynchronize();  // the alignment kernel's results are complete
+  const uint32_t count = *(volatile uint32_t*)&L.queue_counts[4];
+  for (uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x; slot < count; slot += gridDim.x * blockDim.x) {
+    const uint32_t item = L.queue_pass[slot];
+    const uint32_t t = find_task(L.task_prefix, L.ntask, item);
+    const uint32_t g = L.tasks[t].base + (item - L.task_prefix[t]);
+    L.comp_index[slot] = g;
+    L.comp_lambda[slot] = L.pool.res_lambda[g];
+    L.comp_ham[slot] = (L.pool.res_ham[g] & ((1u << kPostMethod) - 1)) | (uint32_t(L.pool.res_status[g] >> 2) << kPostMethod);
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    volatile uint32_t* e = L.err_host;
+    e[0] = *L.err_word;
+    e[1] = L.queue_counts[5];
+    e[2] = count;
+  }
+  // the last block to have read the count clears it
+  __shared__ uint32_t s_last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(&L.queue_counts[7], 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (s_last && threadIdx.x < 8) L.queue_counts[threadIdx.x] = 0;
+}
+
 static int g_sm_count = 0;
 static int sm_count() {
   if (g_sm_count == 0) {
@@ -3027,8 +3060,8 @@ static void (*align_kernel(const CompareLaunch& L, size_t smem))(CompareLaunch) 
 }
 
 // The launch sequence of one compare: k_pivot_dots (pivot_blocks > 0), the
-// screen, k_align and the store (store_grid > 0), chained by programmatic
-// dependent launch when the tuning asks for it.
+// screen, k_align and the store (store_grid > 0) or k_collect (do_store 0),
+// chained by programmatic dependent launch when the tuning asks for it.
 static void launch_chain(const CompareLaunch& L, cudaStream_t st, cudaEvent_t* ev, uint32_t screen_blocks,
                          uint32_t pivot_blocks, uint32_t store_grid, void (*kalign)(CompareLaunch), size_t asmem) {
   if (ev) cudaEventRecord(ev[0], st);
@@ -3074,6 +3107,11 @@ static void launch_chain(const CompareLaunch& L, cudaStream_t st, cudaEvent_t* e
     cfg.blockDim = dim3(kStoreThreads);
     cfg.dynamicSmemBytes = 0;
     cudaLaunchKernelEx(&cfg, k_store, L);
+  } else if (!L.do_store) {
+    cfg.gridDim = dim3(std::min<uint32_t>((L.total_items + 255) / 256, uint32_t(sm_count()) * 2u));
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = 0;
+    cudaLaunchKernelEx(&cfg, k_collect, L);
   }
   if (ev) cudaEventRecord(ev[3], st);
 }

@@ -129,13 +129,13 @@ class CompareContext:
 
     def compare(self, center: int, kdist_cutoff: float, greedy: bool = True):
         """The map: per-raw (lambda, hamming or UINT32_MAX, skipped)."""
-        lam = np.zeros(self.n, np.float64)
-        ham = np.zeros(self.n, np.uint32)
-        skp = np.zeros(self.n, np.uint8)
+        lam = np.empty(self.n, np.float64)
+        ham = np.empty(self.n, np.uint32)
+        skp = np.empty(self.n, np.bool_)
         cnt = CountersC()
         check(lib().dgpu_compare(self.h, int(center), float(kdist_cutoff), int(bool(greedy)), ptr(lam), ptr(ham),
                                  ptr(skp), C.byref(cnt)))
-        return lam, ham, skp.astype(bool), _counters(cnt)
+        return lam, ham, skp, _counters(cnt)
 
     def b_compare_parallel(self, center: int, cluster_i: int, kdist_cutoff: float, greedy: bool = True):
         """Map + store: the stored comparisons in ascending raw order."""
