@@ -2452,6 +2452,87 @@ __device__ __forceinline__ void gapless_codes(int lane, const uint8_t* sc, int l
   }
 }
 
+// Whether every alignment of two sequences of L bases other than the plain
+// diagonal one scores below it under match 5, mismatch -4, gap -8 (so the DP
+// would walk the diagonal), shown without the DP for up to three mismatches.
+// *ham gets the mismatches. s1 and s2 are the staged codes 1..4.
+//
+// Count what an alignment loses against five points a base: 9 a mismatch, and 5
+// a base left out. The diagonal loses 9 m. Another path leaves the diagonal in
+// stretches; one that leaves and returns loses at least 21 in gaps, one at an
+// end of the sequences 13 per diagonal it is away, one that never returns 5
+// per diagonal and 8 per gap. So with m <= 3 a stretch pays only if
+//  * it never returns, is at most 5 diagonals away and has at most 2 gaps: but
+//    then one of the four or more whole words of 32 rows lies on one diagonal,
+//    and every word of every such diagonal has ten or more mismatches;
+//  * it spans mismatches 1-3 inside, on a neighbouring diagonal, without a
+//    mismatch of its own;
+//  * it runs from an end over two of the mismatches, on a neighbouring
+//    diagonal, without a mismatch of its own; or over all three there with at
+//    most one, or two diagonals away with none (the rows it leaves out, two,
+//    may hide as many that match neither diagonal).
+// Rows that such a stretch surely covers are tested for the mismatches that
+// would spoil it; where they do not show up, the answer is no and the DP runs.
+// The late calls of a denoising meet mostly such pairs (98 % of those that take
+// the DP have up to three mismatches), and a call waits for its slowest pair.
+__device__ bool diagonal_is_best(int lane, const uint8_t* s1, const uint8_t* s2, int L, uint32_t* ham) {
+  if (L < 128 || L > 512) return false;
+  const int word = lane & 15, neg = lane >> 4;  // lanes 16..31 take the diagonals below
+  uint32_t a0 = 0, a1 = 0, b0 = 0, b1 = 0, m = 0;
+  int pos[3] = {0, 0, 0};
+  for (int w = 0; 32 * w < L; ++w) {
+    const int p = 32 * w + lane;
+    const unsigned u = p < L ? s1[p] - 1u : 0u, v = p < L ? s2[p] - 1u : 0u;
+    uint32_t mm = __ballot_sync(FULL, u != v);
+    m += __popc(mm);
+    if (m > 3) return false;
+    for (; mm; mm &= mm - 1) {
+      pos[0] = pos[1];
+      pos[1] = pos[2];
+      pos[2] = 32 * w + __ffs(mm) - 1;
+    }
+    const uint32_t w0 = __ballot_sync(FULL, u & 1u), w1 = __ballot_sync(FULL, u & 2u);
+    const uint32_t v0 = __ballot_sync(FULL, v & 1u), v1 = __ballot_sync(FULL, v & 2u);
+    if (word == w) {
+      a0 = w0;
+      a1 = w1;
+      b0 = v0;
+      b1 = v1;
+    }
+  }
+  *ham = m;
+  if (m == 0) return true;
+  // x[d - 1]: the rows of this lane's word that mismatch d diagonals away
+  const int nb = (lane & 16) | ((word + (neg ? 15 : 1)) & 15);  // the word before or after
+  const uint32_t n0 = __shfl_sync(FULL, b0, nb), n1 = __shfl_sync(FULL, b1, nb);
+  uint32_t x1 = 0, x2 = 0;
+  bool good = true;
+#pragma unroll
+  for (int d = 1; d <= 5; ++d) {
+    const uint32_t c0 = neg ? __funnelshift_l(n0, b0, d) : __funnelshift_r(b0, n0, d);
+    const uint32_t c1 = neg ? __funnelshift_l(n1, b1, d) : __funnelshift_r(b1, n1, d);
+    const int rows = min(max((neg ? L : L - d) - 32 * word, 0), 32);
+    uint32_t x = ((a0 ^ c0) | (a1 ^ c1)) & (rows == 32 ? FULL : (1u << rows) - 1u);
+    if (neg && word == 0) x &= FULL << d;
+    good = good && (32 * word + 32 > L || __popc(x) >= 10);
+    if (d == 1) x1 = x;
+    if (d == 2) x2 = x;
+  }
+  if (!__all_sync(FULL, good)) return false;
+  if (m == 1) return true;
+  // whether both sides have at least k of x's rows in [lo, hi]
+  auto rows_of = [&](uint32_t x, int lo, int hi, uint32_t k) {
+    const int f = min(max(lo - 32 * word, 0), 32), e = min(max(hi + 1 - 32 * word, 0), 32);
+    const uint32_t upto_e = e == 32 ? FULL : (1u << e) - 1u, upto_f = f == 32 ? FULL : (1u << f) - 1u;
+    const uint32_t c = __reduce_add_sync(FULL, uint32_t(__popc(x & upto_e & ~upto_f)) << (16 * neg));
+    return (c & 0xffffu) >= k && (c >> 16) >= k;
+  };
+  if (m == 2) return rows_of(x1, 1, pos[2] - 1, 1) && rows_of(x1, pos[1] + 1, L - 2, 1);
+  return rows_of(x1, pos[0] + 1, pos[2] - 1, 1) && rows_of(x1, 1, pos[1] - 1, 1) &&
+         rows_of(x1, pos[1] + 1, L - 2, 1) && rows_of(x1, 2, pos[2] - 2, 2) && rows_of(x1, pos[0] + 2, L - 3, 2) &&
+         rows_of(x1 & x2, 2, pos[2] - 2, 3) && rows_of(x1 & x2, pos[0] + 2, L - 3, 3);
+}
+
 // align_pair for launches whose geometry lets every pair take the strip
 // aligner (NwGeom::strip_c). planes: the warp's pointer words in global memory
 // when they do not stay in shared memory.
@@ -2467,9 +2548,11 @@ __device__ __forceinline__ PairResult align_pair_strip(int lane, const KParams& 
   __syncwarp();
   PairResult R{true, AM_NONE, 0u, lg, S.tcode, S.fidx, stage_q ? S.qual : qg};
   uint32_t ham = 0;
-  if (takes_gapless(lane, kp, S.s1, lc, S.s2, lg, kdist, &ham)) {
+  const bool gapless = takes_gapless(lane, kp, S.s1, lc, S.s2, lg, kdist, &ham);
+  if (gapless || (FORMS == kFormsStrip1 && lc == lg && kp.match == 5 && kp.mismatch == -4 && kp.gap == -8 &&
+                  diagonal_is_best(lane, S.s1, S.s2, lg, &ham))) {
     gapless_codes(lane, S.s1, lc, S.s2, lg, S.tcode);
-    R.method = AM_GAPLESS;
+    R.method = gapless ? AM_GAPLESS : (kp.vectorized ? AM_VECTORIZED : AM_ENDSFREE);
   } else {
     const bool homo = FORMS != kFormsStrip1 && kp.homo_gap != kp.gap && kp.homo_gap <= 0;
     uint2* planes = geom.strip_smem ? S.stage : reinterpret_cast<uint2*>(scratch);
