@@ -211,7 +211,7 @@ __device__ __forceinline__ bool strip_align(int lane, int len1, int len2, int ma
   const int nl = (W + N - 1) / N;
   const int lc = min(lane, nl - 1);  // idle lanes read what the last one does
   const int ol = o_lo + N * lc;
-  int V[N], LB[N], Y[N];
+  int V[N], LB[N], Y[N], CL[HOMO ? N : 1];  // values; band-edge marks; column codes and gap costs
   // before its first row a cell holds its value on row 0 (o >= 0) or column 0
   {
     int c1[N], c2[N];
@@ -257,7 +257,13 @@ __device__ __forceinline__ bool strip_align(int lane, int len1, int len2, int ma
   using Fast = std::integral_constant<bool, false>;
   int x = x_at(-lc, Slow{});  // row r - lc = 1 - lc
 #pragma unroll
-  for (int k = 0; k < N; ++k) Y[k] = y_at(ol - lc + k, Slow{});
+  for (int k = 0; k < N; ++k) {
+    Y[k] = y_at(ol - lc + k, Slow{});
+    if (HOMO) {
+      CL[k] = (Y[k] & 16) ? -hgap : -gap;
+      Y[k] &= 15;
+    }
+  }
   // N rows from row count r on; cell k of row u reads column slot (k + u) % N
   auto rows = [&](int r, auto slow) {
     constexpr bool SLOW = decltype(slow)::value;
@@ -271,9 +277,8 @@ __device__ __forceinline__ bool strip_align(int lane, int len1, int len2, int ma
       // without runs both gap costs are the same constant
       const int wa = match + cu + (HOMO ? 0 : -gap), wb = mismatch + cu + (HOMO ? 0 : -gap);
       auto cell = [&](int k, int left, int up, bool up_late) -> int {
-        const int y = Y[(k + u) % N];
-        const int cl = HOMO ? ((y & 16) ? -hgap : -gap) : -gap;
-        const int w = (HOMO ? (y & 15) : y) == xc ? wa : wb;
+        const int cl = HOMO ? CL[(k + u) % (HOMO ? N : 1)] : -gap;
+        const int w = Y[(k + u) % N] == xc ? wa : wb;
         const int dg = HOMO ? V[k] + w + cl : V[k] + w;
         if (SLOW) {
           if (i + ol + k == len2) up += cu;  // free on the last column
@@ -294,7 +299,8 @@ __device__ __forceinline__ bool strip_align(int lane, int len1, int len2, int ma
       const int ub = __shfl_down_sync(FULL, V[0], 1);
 #pragma unroll
       for (int k = C; k < N; ++k) left = V[k] = cell(k, left, k + 1 < N ? V[(k + 1) % N] : ub, k + 1 == N);
-      Y[u] = yn;
+      Y[u] = HOMO ? yn & 15 : yn;
+      if (HOMO) CL[u % (HOMO ? N : 1)] = (yn & 16) ? -hgap : -gap;
       x = xn;
       if (++cnt == RPW) {
         *out = make_uint2(accD, accL);
