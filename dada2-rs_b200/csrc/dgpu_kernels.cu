@@ -362,7 +362,8 @@ __global__ void __launch_bounds__(kScreenWarps * 32, 4) k_screen(CompareLaunch L
   __shared__ uint32_t s_prefix[kScreenSmemTasks + 1];
   __shared__ uint32_t s_base[kScreenSmemTasks], s_center[kScreenSmemTasks], s_creads[kScreenSmemTasks];
   __shared__ double s_cutoff[kScreenSmemTasks];
-  __shared__ uint32_t s_cluster[kScreenSmemTasks];
+  __shared__ uint32_t s_cluster[kScreenSmemTasks], s_clen[kScreenSmemTasks];
+  __shared__ uint8_t s_csat[kScreenSmemTasks];
   // direct store: this block's screened and shrouded raws per task
   __shared__ uint32_t s_ctr[2 * kScreenSmemTasks];
   const bool direct = L.direct != 0;
@@ -384,6 +385,8 @@ __global__ void __launch_bounds__(kScreenWarps * 32, 4) k_screen(CompareLaunch L
         s_creads[t] = T.center_reads;
         s_cutoff[t] = T.cutoff;
         s_cluster[t] = T.cluster;
+        s_clen[t] = L.pool.len[T.center];
+        s_csat[t] = L.pool.sat[T.center];
       }
     }
     __syncthreads();
@@ -403,7 +406,8 @@ __global__ void __launch_bounds__(kScreenWarps * 32, 4) k_screen(CompareLaunch L
     const uint32_t item = chunk + lane;
     const bool valid = uint32_t(lane) < CH && item < L.total_items;
     uint32_t t = 0, g = 0, c = 0, ccl = 0, tbase = 0;
-    bool skip = false, bounded = false, pivot_raw = false, cl_fits = false;
+    int lc = 0, lg = 0;
+    bool skip = false, bounded = false, pivot_raw = false, cl_fits = false, sat_c = false, sat_g = false;
     if (valid) {
       uint32_t creads;
       if (tasks_smem) {
@@ -412,18 +416,29 @@ __global__ void __launch_bounds__(kScreenWarps * 32, 4) k_screen(CompareLaunch L
         c = s_center[t];
         creads = s_creads[t];
         ccl = s_cluster[t];
+        lc = int(s_clen[t]);
+        sat_c = s_csat[t] != 0;
       } else {
         t = find_task(L.task_prefix, L.ntask, item);
         tbase = L.tasks[t].base;
         c = L.tasks[t].center;
         creads = L.tasks[t].center_reads;
         ccl = L.tasks[t].cluster;
+        lc = int(L.pool.len[c]);
+        sat_c = L.pool.sat[c] != 0;
       }
       const uint32_t t0 = tasks_smem ? s_prefix[t] : L.task_prefix[t];
       const uint32_t tn = (tasks_smem ? s_prefix[t + 1] : L.task_prefix[t + 1]) - t0;
       g = tbase + (item - t0);
       cl_fits = ccl < tn;  // cluster indices of a whole sample stay below its raw count
+      // everything the raw's fate may need is loaded at once: one round trip,
+      // then one for the pivot's dot (taken one after the other as each test
+      // passed, they were five)
+      const uint32_t reads = L.pool.reads[g];
       bool locked = L.pool.lock[g] != 0;
+      lg = int(L.pool.len[g]);
+      sat_g = L.pool.sat[g] != 0;
+      const uint32_t pc = pivot ? L.pool.piv_cl[g] : kNoPivot, pd = pivot ? L.pool.piv_dot[g] : 0u;
       if (!locked && nlock4) {
         for (uint32_t q = 0; q < nlock4; ++q) {
           const uint4 x = s_lock[q];
@@ -431,7 +446,7 @@ __global__ void __launch_bounds__(kScreenWarps * 32, 4) k_screen(CompareLaunch L
         }
         if (locked) L.pool.lock[g] = 1;
       }
-      skip = kp.greedy && (L.pool.reads[g] > creads || locked);
+      skip = kp.greedy && (reads > creads || locked);
       if (pivot && !skip) {
         // Exact exclusion without reading the raw's profile. For non-negative
         // count vectors min(c, r) <= min(c, p) + r - min(r, p) elementwise, so
@@ -441,16 +456,12 @@ __global__ void __launch_bounds__(kScreenWarps * 32, 4) k_screen(CompareLaunch L
         // too, so a bound kdist above the cutoff means the exact one is above
         // it as well: the raw is shrouded (src/nwalign.rs:1295-1301). Raws or
         // centers with a saturated count take the exact path and never this.
-        const int lc = int(L.pool.len[c]), lg = int(L.pool.len[g]);
-        pivot_raw = cl_fits && !L.pool.sat[g] && !L.pool.sat[c] && lc >= K && lg >= K;
-        if (pivot_raw && L.cdot_ready) {
-          const uint32_t pc = L.pool.piv_cl[g];
-          if (pc < ccl) {
-            const int minl = lc < lg ? lc : lg;
-            const uint32_t ub = L.pool.cdot[tbase + pc] + uint32_t(lg - K + 1) - L.pool.piv_dot[g];
-            const double kd_lb = 1.0 - double(ub) / double(minl - K + 1);
-            bounded = kd_lb > (tasks_smem ? s_cutoff[t] : L.tasks[t].cutoff);
-          }
+        pivot_raw = cl_fits && !sat_g && !sat_c && lc >= K && lg >= K;
+        if (pivot_raw && L.cdot_ready && pc < ccl) {
+          const int minl = lc < lg ? lc : lg;
+          const uint32_t ub = L.pool.cdot[tbase + pc] + uint32_t(lg - K + 1) - pd;
+          const double kd_lb = 1.0 - double(ub) / double(minl - K + 1);
+          bounded = kd_lb > (tasks_smem ? s_cutoff[t] : L.tasks[t].cutoff);
         }
       }
     }
@@ -563,7 +574,7 @@ __global__ void __launch_bounds__(kScreenWarps * 32, 4) k_screen(CompareLaunch L
     // saturates, so the result is the reference's in every case. One item at a
     // time by the whole warp: each window of the raw contributes 1 when its rank
     // among equal windows of the raw is below the center's count of that k-mer.
-    const bool maybe_ovf = need && L.pool.sat[g] && L.pool.sat[c];
+    const bool maybe_ovf = need && sat_g && sat_c;
     (void)myovf;
     uint32_t ovf_mask = __ballot_sync(FULL, maybe_ovf);
     while (ovf_mask) {
@@ -608,7 +619,6 @@ __global__ void __launch_bounds__(kScreenWarps * 32, 4) k_screen(CompareLaunch L
       if (!bounded && !skip) {
         double kdist = 0.0;
         if (kp.use_kmers) {
-          const int lc = int(L.pool.len[c]), lg = int(L.pool.len[g]);
           const int minl = lc < lg ? lc : lg;
           kdist = 1.0 - double(mydot) / double(minl - K + 1);
           shroud = kdist > (tasks_smem ? s_cutoff[t] : L.tasks[t].cutoff);
