@@ -103,6 +103,7 @@ struct NwGeom {
   int32_t vec_nrow;    // 2*lmax+1
   int32_t rm_pairs;    // bound on offset pairs of the row-major band (ceil(W/2))
   int32_t nwarps;      // resident warps of the persistent NW kernels
+  int32_t late_warps;  // those of a direct call's (at most nwarps)
   size_t vec_scratch;  // bytes per warp (pointer matrix)
   size_t rm_scratch;   // bytes per warp (pointer bit planes)
   int32_t forms;       // the aligner forms a compare launch can reach (kForms*)

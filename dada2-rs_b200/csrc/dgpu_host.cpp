@@ -790,7 +790,8 @@ struct Pool {
     // (at most 4 groups) for the register form
     geom.vec_scratch = vec_possible ? align16(size_t(geom.vec_nrow) * std::max<size_t>(size_t(geom.vec_ncol), 32)) : 0;
     geom.rm_scratch = rm_possible ? align16(size_t(2 * lmax + 1) * 2 * kb * 4) : 0;
-    geom.nwarps = sms * tuning_for(lmax).align_ctas_per_sm * kNwWarps;
+    geom.nwarps = sms * kAlignCtasPerSm * kNwWarps;
+    geom.late_warps = sms * tuning_for(lmax).align_ctas_per_sm * kNwWarps;
     // the forms k_align can reach: the strip aligner alone when it takes every
     // pair (see strip_takes), one diagonal per strip when no pair needs more
     geom.forms = rm_possible && !vec_possible ? kFormsRm : kFormsAll;
