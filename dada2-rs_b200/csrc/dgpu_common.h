@@ -287,9 +287,20 @@ struct CompareLaunch {
   // cdot_ready, total_cl and the table pointers come from *hdr
   const CallHeader* hdr;
 };
+// A call's tables (the upload that starts with its CallHeader) as a kernel
+// parameter, for direct and map calls whose tables fit: no copy precedes the
+// kernels (2.5 us a call). The other calls' kernels take NoTables: 2 kB more
+// of parameters made a graph replay of the 40-sample batch 3 % slower.
+constexpr uint32_t kInlinePack = 2048;
+struct CallTables {
+  alignas(16) uint8_t pack[kInlinePack];
+};
+struct NoTables {};
+// tb: the call's tables when they go up as a parameter, else null.
 // ev (optional): 4 events recorded before the screen and after screen, align
 // and store, for per-kernel device times.
-void launch_compare(const CompareLaunch& L, cudaStream_t st, cudaEvent_t* ev = nullptr);
+void launch_compare(const CompareLaunch& L, cudaStream_t st, const CallTables* tb = nullptr,
+                    cudaEvent_t* ev = nullptr);
 // The screen's chunk size for a call of `total` items (launch_compare's rule).
 uint32_t compare_screen_chunk(uint32_t total, uint32_t screen_blocks_per_sm, uint32_t screen_chunk_max);
 // Captures the compare sequence on `st` as a graph for replay with L.hdr set:

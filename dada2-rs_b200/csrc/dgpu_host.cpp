@@ -502,6 +502,7 @@ struct Slot {
   DBuf<uint8_t> scratch;
   DBuf<uint8_t> dpack;  // tasks | task prefix | store map of the current launch
   HBuf<uint8_t> hpack;  // its pinned staging copy (one upload per launch)
+  CallTables tables{};  // the same as a kernel parameter
   HBuf<uint32_t> blk_counters, err_host;
   HBuf<double> task_self;
   HBuf<TaskDev> task_stage;
@@ -1009,8 +1010,18 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_di
     H.o_clp = uint32_t(o_clp);
     H.o_map = uint32_t(o_map);
   }
-  CUDA_TRY(cudaMemcpyAsync(dpack.p, hpack.h, pack_bytes, cudaMemcpyHostToDevice, st));
-  count_h2d(pack_bytes);
+  const uint64_t every = g_stats.timing_every.load();
+  const bool timing = every != 0 && g_stats.call_seq.fetch_add(1) % every == 0;
+  const bool replay = do_store && !timing && total > 0 && Q.replay_graphs && compare_graphs_on() && !graphs_failed;
+  // direct and map calls launched one kernel at a time take their tables as a
+  // parameter when these fit
+  const bool inline_tables = (direct || !do_store) && !replay && pack_bytes <= kInlinePack;
+  if (inline_tables) {
+    std::memcpy(tables.pack, hpack.h, pack_bytes);
+  } else {
+    CUDA_TRY(cudaMemcpyAsync(dpack.p, hpack.h, pack_bytes, cudaMemcpyHostToDevice, st));
+    count_h2d(pack_bytes);
+  }
   CompareLaunch L;
   std::memset(&L, 0, sizeof L);  // padding too: graph_key compares the bytes
   L.pool = Q.view();
@@ -1049,10 +1060,8 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_di
   L.cdot_ready = cdot_ready ? 1u : 0u;
   L.task_cl_prefix = reinterpret_cast<const uint32_t*>(dpack.p + o_clp);
   L.total_cl = cdot_ready ? total_cl : 0u;
-  const uint64_t every = g_stats.timing_every.load();
-  const bool timing = every != 0 && g_stats.call_seq.fetch_add(1) % every == 0;
   bool launched = false;
-  if (do_store && !timing && total > 0 && Q.replay_graphs && compare_graphs_on() && !graphs_failed) {
+  if (replay) {
     // Replay a captured graph of the launch sequence: one submission instead
     // of three or four, which the launch slots' threads otherwise contend
     // for in the driver. Its kernels take this call's values from the
@@ -1106,7 +1115,7 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_di
       launched = true;
     }
   }
-  if (!launched) launch_compare(L, st, timing ? ev : nullptr);
+  if (!launched) launch_compare(L, st, inline_tables ? &tables : nullptr, timing ? ev : nullptr);
   CUDA_TRY(cudaGetLastError());
   auto t0 = Clock::now();
   // Poll and yield rather than block in the driver's spin: the launch slots'

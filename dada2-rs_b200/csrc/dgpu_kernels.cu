@@ -282,9 +282,11 @@ __device__ __forceinline__ uint32_t mismatch_word(const uint8_t* a, const uint8_
 
 // Lean streaming screen: greedy skip, profile dot product, strict cutoff
 // (src/cluster.rs:295-298, src/kmers.rs:254-269, src/nwalign.rs:1299).
-// A graph replay's per-call values (CompareLaunch::hdr) into the kernel's
-// own copy of the launch parameters.
-__device__ __forceinline__ void load_call(CompareLaunch& L) {
+// The per-call values of a graph replay (CompareLaunch::hdr) or of tables that
+// came as a parameter into the kernel's own copy of the launch parameters.
+template <class Tb>
+__device__ __forceinline__ void load_call(CompareLaunch& L, const Tb& tb) {
+  if constexpr (std::is_same_v<Tb, CallTables>) L.hdr = reinterpret_cast<const CallHeader*>(tb.pack);
   if (!L.hdr) return;
   const CallHeader H = *L.hdr;
   const uint8_t* base = reinterpret_cast<const uint8_t*>(L.hdr);
@@ -309,10 +311,10 @@ __device__ __forceinline__ void load_call(CompareLaunch& L) {
 // sample, cdot[base + i] = the u8 k-mer dot of the task's center with cluster
 // i's center (cl_center[base + i]); the screen's pivot bound reads them. One
 // warp per (task, cluster) item, 16-byte vector loads of both profiles.
-template <int K>
-__global__ void __launch_bounds__(256) k_pivot_dots(CompareLaunch Lp) {
+template <int K, class Tb>
+__global__ void __launch_bounds__(256) k_pivot_dots(CompareLaunch Lp, const __grid_constant__ Tb tb) {
   CompareLaunch L = Lp;
-  load_call(L);
+  load_call(L, tb);
   cudaTriggerProgrammaticLaunchCompletion();  // the screen may start launching
   if (!L.cdot_ready) return;
   constexpr int NK16 = (1 << (2 * K)) / 16;
@@ -342,10 +344,10 @@ __global__ void __launch_bounds__(256) k_pivot_dots(CompareLaunch Lp) {
 // metadata, then the warp streams the raw profiles four at a time against the
 // center profile held in registers. Survivors go to the align queue with their
 // kdist parked in res_lambda.
-template <int K>
-__global__ void __launch_bounds__(kScreenWarps * 32, 4) k_screen(CompareLaunch Lp) {
+template <int K, class Tb>
+__global__ void __launch_bounds__(kScreenWarps * 32, 4) k_screen(CompareLaunch Lp, const __grid_constant__ Tb tb) {
   CompareLaunch L = Lp;
-  load_call(L);
+  load_call(L, tb);
   // every screen block is running: the alignment kernel may start launching
   // (its blocks wait for this grid's results in cudaGridDependencySynchronize)
   cudaTriggerProgrammaticLaunchCompletion();
@@ -2646,10 +2648,11 @@ __device__ __forceinline__ PairResult align_pair(int lane, const KParams& kp, co
 // codes for ACGT input), method choice (src/nwalign.rs:1324-1403), then the
 // gapless alignment or the vectorized / row-major aligner, then lambda.
 // ---------------------------------------------------------------------------
-template <int FORMS>
-__global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(CompareLaunch Lp) {
+template <int FORMS, class Tb>
+__global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(CompareLaunch Lp,
+                                                                          const __grid_constant__ Tb tb) {
   CompareLaunch L = Lp;
-  load_call(L);
+  load_call(L, tb);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cudaTriggerProgrammaticLaunchCompletion();  // the store kernel may start launching
   const KParams& kp = L.kp;
@@ -2920,7 +2923,7 @@ void launch_final_subs(const FinalSubsLaunch& F, cudaStream_t st) {
 // in order gives ascending raw order) with a per-CTA count and counters.
 __global__ void __launch_bounds__(kStoreThreads) k_store(CompareLaunch Lp) {
   CompareLaunch L = Lp;
-  load_call(L);
+  load_call(L, NoTables{});
   if (blockIdx.x >= L.nstore_blocks) return;  // a replayed graph's spare CTAs
   constexpr int IPT = kStoreSpan / kStoreThreads;
   __shared__ uint32_t warp_off[32];
@@ -3053,7 +3056,10 @@ __global__ void __launch_bounds__(kStoreThreads) k_store(CompareLaunch Lp) {
 // outcome follows from the host's own reads and locks. A call over 400,000
 // uniques moves 0.4 MB for its 28,000 pairs, not the 5.2 MB of every raw's
 // entries. Its first block rearms the queue, as k_store's does.
-__global__ void __launch_bounds__(256) k_collect(CompareLaunch L) {
+template <class Tb>
+__global__ void __launch_bounds__(256) k_collect(CompareLaunch Lp, const __grid_constant__ Tb tb) {
+  CompareLaunch L = Lp;
+  load_call(L, tb);
   cudaGridDependencySynchronize();  // the alignment kernel's results are complete
   const uint32_t count = *(volatile uint32_t*)&L.queue_counts[4];
   for (uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x; slot < count; slot += gridDim.x * blockDim.x) {
@@ -3130,11 +3136,12 @@ uint32_t compare_screen_chunk(uint32_t total, uint32_t screen_blocks_per_sm, uin
 // The k_align instance for the forms a launch can reach, with its attributes
 // set once per device (dynamic shared memory above 48 KB, the largest
 // carveout so that kAlignCtasPerSm CTAs fit beside each other).
-static void (*align_kernel(const CompareLaunch& L, size_t smem))(CompareLaunch) {
-  static void (*const forms[4])(CompareLaunch) = {k_align<kFormsAll>, k_align<kFormsStrip1>, k_align<kFormsRm>,
-                                                  k_align<kFormsStrip>};
+template <class Tb>
+static void (*align_kernel(const CompareLaunch& L, size_t smem))(CompareLaunch, Tb) {
+  static void (*const forms[4])(CompareLaunch, Tb) = {k_align<kFormsAll, Tb>, k_align<kFormsStrip1, Tb>,
+                                                      k_align<kFormsRm, Tb>, k_align<kFormsStrip, Tb>};
   const int fi = L.geom.forms;
-  void (*kalign)(CompareLaunch) = forms[fi];
+  void (*kalign)(CompareLaunch, Tb) = forms[fi];
   static std::atomic<int> limit[4][64];
   static std::atomic<uint64_t> carved[4];
   int dev = 0;
@@ -3155,16 +3162,18 @@ static void (*align_kernel(const CompareLaunch& L, size_t smem))(CompareLaunch) 
 // The launch sequence of one compare: k_pivot_dots (pivot_blocks > 0), the
 // screen, k_align and the store (store_grid > 0) or k_collect (do_store 0),
 // chained by programmatic dependent launch when the tuning asks for it.
-static void launch_chain(const CompareLaunch& L, cudaStream_t st, cudaEvent_t* ev, uint32_t screen_blocks,
-                         uint32_t pivot_blocks, uint32_t store_grid, void (*kalign)(CompareLaunch), size_t asmem) {
+template <class Tb>
+static void launch_chain(const CompareLaunch& L, const Tb& tb, cudaStream_t st, cudaEvent_t* ev,
+                         uint32_t screen_blocks, uint32_t pivot_blocks, uint32_t store_grid,
+                         void (*kalign)(CompareLaunch, Tb), size_t asmem) {
   if (ev) cudaEventRecord(ev[0], st);
   if (pivot_blocks > 0) {
     switch (L.kp.kmer_size) {
-      case 3: k_pivot_dots<3><<<pivot_blocks, 256, 0, st>>>(L); break;
-      case 4: k_pivot_dots<4><<<pivot_blocks, 256, 0, st>>>(L); break;
-      case 5: k_pivot_dots<5><<<pivot_blocks, 256, 0, st>>>(L); break;
-      case 6: k_pivot_dots<6><<<pivot_blocks, 256, 0, st>>>(L); break;
-      default: k_pivot_dots<7><<<pivot_blocks, 256, 0, st>>>(L); break;
+      case 3: k_pivot_dots<3, Tb><<<pivot_blocks, 256, 0, st>>>(L, tb); break;
+      case 4: k_pivot_dots<4, Tb><<<pivot_blocks, 256, 0, st>>>(L, tb); break;
+      case 5: k_pivot_dots<5, Tb><<<pivot_blocks, 256, 0, st>>>(L, tb); break;
+      case 6: k_pivot_dots<6, Tb><<<pivot_blocks, 256, 0, st>>>(L, tb); break;
+      default: k_pivot_dots<7, Tb><<<pivot_blocks, 256, 0, st>>>(L, tb); break;
     }
   }
   // Programmatic dependent launch: the alignment and store kernels, and the
@@ -3181,12 +3190,12 @@ static void launch_chain(const CompareLaunch& L, cudaStream_t st, cudaEvent_t* e
   cfg.gridDim = dim3(screen_blocks);
   cfg.blockDim = dim3(kScreenWarps * 32);
   switch (L.kp.kmer_size) {
-    case 3: cudaLaunchKernelEx(&cfg, k_screen<3>, L); break;
-    case 4: cudaLaunchKernelEx(&cfg, k_screen<4>, L); break;
-    case 5: cudaLaunchKernelEx(&cfg, k_screen<5>, L); break;
-    case 6: cudaLaunchKernelEx(&cfg, k_screen<6>, L); break;
-    case 7: cudaLaunchKernelEx(&cfg, k_screen<7>, L); break;
-    default: cudaLaunchKernelEx(&cfg, k_screen<8>, L); break;
+    case 3: cudaLaunchKernelEx(&cfg, k_screen<3, Tb>, L, tb); break;
+    case 4: cudaLaunchKernelEx(&cfg, k_screen<4, Tb>, L, tb); break;
+    case 5: cudaLaunchKernelEx(&cfg, k_screen<5, Tb>, L, tb); break;
+    case 6: cudaLaunchKernelEx(&cfg, k_screen<6, Tb>, L, tb); break;
+    case 7: cudaLaunchKernelEx(&cfg, k_screen<7, Tb>, L, tb); break;
+    default: cudaLaunchKernelEx(&cfg, k_screen<8, Tb>, L, tb); break;
   }
   if (ev) cudaEventRecord(ev[1], st);
   cfg.numAttrs = L.pdl ? 1 : 0;
@@ -3197,7 +3206,7 @@ static void launch_chain(const CompareLaunch& L, cudaStream_t st, cudaEvent_t* e
   cfg.gridDim = dim3(late ? L.geom.late_warps / kNwWarps : L.geom.nwarps / kNwWarps);
   cfg.blockDim = dim3(kNwWarps * 32);
   cfg.dynamicSmemBytes = asmem;
-  cudaLaunchKernelEx(&cfg, kalign, L);
+  cudaLaunchKernelEx(&cfg, kalign, L, tb);
   if (ev) cudaEventRecord(ev[2], st);
   if (store_grid > 0) {
     cfg.gridDim = dim3(store_grid);
@@ -3208,12 +3217,12 @@ static void launch_chain(const CompareLaunch& L, cudaStream_t st, cudaEvent_t* e
     cfg.gridDim = dim3(std::min<uint32_t>((L.total_items + 255) / 256, uint32_t(sm_count()) * 2u));
     cfg.blockDim = dim3(256);
     cfg.dynamicSmemBytes = 0;
-    cudaLaunchKernelEx(&cfg, k_collect, L);
+    cudaLaunchKernelEx(&cfg, k_collect<Tb>, L, tb);
   }
   if (ev) cudaEventRecord(ev[3], st);
 }
 
-void launch_compare(const CompareLaunch& L0, cudaStream_t st, cudaEvent_t* ev) {
+void launch_compare(const CompareLaunch& L0, cudaStream_t st, const CallTables* tb, cudaEvent_t* ev) {
   if (L0.total_items == 0) return;
   const int sms = sm_count();
   const uint32_t bps = (L0.screen_blocks_per_sm >= 1 && L0.screen_blocks_per_sm <= 4) ? L0.screen_blocks_per_sm : 4u;
@@ -3228,17 +3237,19 @@ void launch_compare(const CompareLaunch& L0, cudaStream_t st, cudaEvent_t* ev) {
                           ? std::min<uint32_t>((L.total_cl + 7) / 8, uint32_t(sms) * 8u)
                           : 0u;
   const size_t asm_ = err_smem_bytes(L.kp.ncol) + size_t(kNwWarps) * align_smem_per_warp(L.geom);
-  launch_chain(L, st, ev, blocks, pb, L.do_store && !L.direct ? L.nstore_blocks : 0u, align_kernel(L, asm_), asm_);
+  const uint32_t store = L.do_store && !L.direct ? L.nstore_blocks : 0u;
+  if (tb) launch_chain(L, *tb, st, ev, blocks, pb, store, align_kernel<CallTables>(L, asm_), asm_);
+  else launch_chain(L, NoTables{}, st, ev, blocks, pb, store, align_kernel<NoTables>(L, asm_), asm_);
 }
 
 int capture_compare_graph(const CompareLaunch& L, cudaStream_t st, uint32_t screen_grid, bool pivot_dots,
                           uint32_t store_grid, cudaGraph_t* out) {
   const int sms = sm_count();
   const size_t asm_ = err_smem_bytes(L.kp.ncol) + size_t(kNwWarps) * align_smem_per_warp(L.geom);
-  void (*kalign)(CompareLaunch) = align_kernel(L, asm_);  // attributes before the capture
+  void (*kalign)(CompareLaunch, NoTables) = align_kernel<NoTables>(L, asm_);  // attributes before the capture
   cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return int(e);
-  launch_chain(L, st, nullptr, screen_grid, pivot_dots && L.kp.kmer_size <= 7 ? uint32_t(sms) * 8u : 0u,
+  launch_chain(L, NoTables{}, st, nullptr, screen_grid, pivot_dots && L.kp.kmer_size <= 7 ? uint32_t(sms) * 8u : 0u,
                store_grid, kalign, asm_);
   cudaGraph_t g = nullptr;
   e = cudaStreamEndCapture(st, &g);
