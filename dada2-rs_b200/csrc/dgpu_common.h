@@ -215,6 +215,15 @@ void launch_profiles(const uint8_t* seq, const uint32_t* off, const uint32_t* le
 void launch_profiles_sparse(const uint8_t* seq, const uint32_t* off, const uint32_t* len, uint32_t nraw,
                             uint32_t lmax, uint16_t* kidx, uint8_t* kcnt, uint32_t* knum, uint8_t* sat,
                             cudaStream_t st);
+// A call's tables (the upload that starts with its CallHeader) as a kernel
+// parameter, for direct and map calls whose tables fit: no copy precedes the
+// kernels (2.5 us a call). The other calls' kernels take NoTables: 2 kB more
+// of parameters made a graph replay of the 40-sample batch 3 % slower.
+constexpr uint32_t kInlinePack = 2048;
+struct CallTables {
+  alignas(16) uint8_t pack[kInlinePack];
+};
+struct NoTables {};
 // Runs screen/gapless/lambda, both NW kernels and the ordered store for `ntask`
 // tasks; `task_prefix` holds ntask+1 running raw counts.
 struct CompareLaunch {
@@ -286,21 +295,13 @@ struct CompareLaunch {
   // replay and ntask, total_items, screen_chunk, nstore_blocks, pivot,
   // cdot_ready, total_cl and the table pointers come from *hdr
   const CallHeader* hdr;
+  // host pointer, for launch_compare alone: the call's tables when they go up
+  // as a kernel parameter, else null
+  const CallTables* tables;
 };
-// A call's tables (the upload that starts with its CallHeader) as a kernel
-// parameter, for direct and map calls whose tables fit: no copy precedes the
-// kernels (2.5 us a call). The other calls' kernels take NoTables: 2 kB more
-// of parameters made a graph replay of the 40-sample batch 3 % slower.
-constexpr uint32_t kInlinePack = 2048;
-struct CallTables {
-  alignas(16) uint8_t pack[kInlinePack];
-};
-struct NoTables {};
-// tb: the call's tables when they go up as a parameter, else null.
 // ev (optional): 4 events recorded before the screen and after screen, align
 // and store, for per-kernel device times.
-void launch_compare(const CompareLaunch& L, cudaStream_t st, const CallTables* tb = nullptr,
-                    cudaEvent_t* ev = nullptr);
+void launch_compare(const CompareLaunch& L, cudaStream_t st, cudaEvent_t* ev = nullptr);
 // The screen's chunk size for a call of `total` items (launch_compare's rule).
 uint32_t compare_screen_chunk(uint32_t total, uint32_t screen_blocks_per_sm, uint32_t screen_chunk_max);
 // Captures the compare sequence on `st` as a graph for replay with L.hdr set:

@@ -1115,7 +1115,8 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_di
       launched = true;
     }
   }
-  if (!launched) launch_compare(L, st, inline_tables ? &tables : nullptr, timing ? ev : nullptr);
+  L.tables = inline_tables ? &tables : nullptr;
+  if (!launched) launch_compare(L, st, timing ? ev : nullptr);
   CUDA_TRY(cudaGetLastError());
   auto t0 = Clock::now();
   // Poll and yield rather than block in the driver's spin: the launch slots'

@@ -1,15 +1,17 @@
 // CUDA kernels of the dada compare step (sm_100a).
 //
-//   k_profiles  -- K1: dense saturating u8 k-mer counts per unique (src/kmers.rs:79-101)
-//   k_screen    -- K2/K3/K6: greedy skip, k-mer screen, ordered-k-mer distance, gapless
-//                  alignment and the FP64 lambda product, one warp per (center, raw)
-//                  (src/cluster.rs:279-330, src/nwalign.rs:1244-1327, src/pval.rs:253-320)
-//   k_nw_vec    -- K4: replica of the rolling i16 anti-diagonal aligner + traceback
-//                  (src/nwalign.rs:665-1140), one warp per pair, persistent
-//   k_nw_rm     -- K5: the row-major i32 ends-free / homopolymer aligner
-//                  (src/nwalign.rs:336-528) evaluated as an anti-diagonal wavefront,
-//                  one warp per pair, persistent
-//   k_store     -- K7: ordered store + e_minmax update + counters (src/cluster.rs:351-397)
+//   k_profiles   -- dense saturating u8 k-mer counts per unique (src/kmers.rs:79-101)
+//   k_pivot_dots -- the new centers' k-mer dots with the earlier ones, for the screen's bound
+//   k_screen     -- greedy skip and k-mer screen of every unique against its sample's
+//                   center (src/cluster.rs:279-330, src/nwalign.rs:1244-1310)
+//   k_align      -- the pairs that pass: ordered-k-mer distance, gapless or banded
+//                   alignment (the strip aligner, dgpu_strip.cuh; older forms where
+//                   its rule rules it out) and the FP64 lambda product, one warp per
+//                   pair (src/nwalign.rs:336-1140, src/pval.rs:253-320); in late calls
+//                   also the store
+//   k_store      -- ordered store + e_minmax update + counters (src/cluster.rs:351-397)
+//   k_collect    -- the aligned pairs of a call without a store
+//   k_final_subs -- realignment to the final centers and transition counts
 //
 // Built with --fmad=false: the FP64 product and the k-mer distances must round
 // exactly like the reference's separately-rounded operations.
@@ -3201,7 +3203,8 @@ static void launch_chain(const CompareLaunch& L, const Tb& tb, cudaStream_t st, 
   cfg.numAttrs = L.pdl ? 1 : 0;
   // A late call's few pairs need few blocks, and each block costs the other
   // streams' kernels room; a call that aligns most uniques fills the SMs
-  // (24,908 pairs of 250 nt: 0.67 ms with two blocks per SM, 0.35 with four).
+  // (a call of 24,908 pairs of 250 nt: 0.97 ms with two blocks per SM, 0.53 with
+  // four).
   const bool late = L.do_store && store_grid == 0;
   cfg.gridDim = dim3(late ? L.geom.late_warps / kNwWarps : L.geom.nwarps / kNwWarps);
   cfg.blockDim = dim3(kNwWarps * 32);
@@ -3222,7 +3225,7 @@ static void launch_chain(const CompareLaunch& L, const Tb& tb, cudaStream_t st, 
   if (ev) cudaEventRecord(ev[3], st);
 }
 
-void launch_compare(const CompareLaunch& L0, cudaStream_t st, const CallTables* tb, cudaEvent_t* ev) {
+void launch_compare(const CompareLaunch& L0, cudaStream_t st, cudaEvent_t* ev) {
   if (L0.total_items == 0) return;
   const int sms = sm_count();
   const uint32_t bps = (L0.screen_blocks_per_sm >= 1 && L0.screen_blocks_per_sm <= 4) ? L0.screen_blocks_per_sm : 4u;
@@ -3238,7 +3241,7 @@ void launch_compare(const CompareLaunch& L0, cudaStream_t st, const CallTables* 
                           : 0u;
   const size_t asm_ = err_smem_bytes(L.kp.ncol) + size_t(kNwWarps) * align_smem_per_warp(L.geom);
   const uint32_t store = L.do_store && !L.direct ? L.nstore_blocks : 0u;
-  if (tb) launch_chain(L, *tb, st, ev, blocks, pb, store, align_kernel<CallTables>(L, asm_), asm_);
+  if (L.tables) launch_chain(L, *L.tables, st, ev, blocks, pb, store, align_kernel<CallTables>(L, asm_), asm_);
   else launch_chain(L, NoTables{}, st, ev, blocks, pb, store, align_kernel<NoTables>(L, asm_), asm_);
 }
 

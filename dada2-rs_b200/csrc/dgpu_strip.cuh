@@ -176,8 +176,8 @@ __device__ __forceinline__ bool strip_traceback(int lane, int len1, int len2, in
 // cell per lane and anti-diagonal, as this replaces, cost a shuffle, the
 // pointer's two ballots and the position's costs for every 32 cells: a call
 // aligning 4,672 pairs of 1,400-1,550 nt (band 32, homopolymer gaps) went from
-// 5.7 to 1.7 ms, one aligning 24,908 pairs of 250 nt (band 16) from 1.4 to
-// 0.8 ms, and one of 4 such pairs from 51 to 30 us.
+// 5.0 to 1.15 ms, one aligning 24,908 pairs of 250 nt (band 16) from 1.8 to
+// 0.53 ms, and one of 4 such pairs from 51 to 30 us.
 //
 // Values are kept less the gap costs of their row and column (H = V - sum of
 // gl over 1..j - sum of gu over 1..i): the two gap moves then cost nothing,
