@@ -281,6 +281,7 @@ struct CompareLaunch {
   // halves. A call that queues more than kPostMax pairs posts its head only
   // and aligns none: the host makes the call again with the store kernel.
   uint32_t direct;
+  uint32_t many_slots;  // the sample's next call may run on another stream
   uint32_t* task_ctr;
   uint64_t* post;
   // direct: the raws locked since the tables' last call (at most kLockListMax);

@@ -1048,6 +1048,7 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_di
   L.direct = direct ? direct_seq : 0u;
   L.lock_list = reinterpret_cast<const uint32_t*>(dpack.p + o_lock);
   L.nlock = nlock;
+  L.many_slots = Q.slots.size() > 1 ? 1u : 0u;
   L.task_ctr = task_ctr.p;
   L.post = post.d;
   L.err_host = err_host.d;
@@ -3869,19 +3870,30 @@ int dgpu_compare(dgpu_ctx* ctx, int center, double kdist_cutoff, int greedy, dou
     }
     nskip += skips;
   };
+  // parts [k, parts) on threads of their own where these can be had
+  const uint32_t parts = n >= 65536 ? std::min(6u, std::max(1u, std::thread::hardware_concurrency() / 2)) : 1u;
+  auto part = [&](uint32_t k) { fill(uint32_t(uint64_t(n) * k / parts), uint32_t(uint64_t(n) * (k + 1) / parts)); };
+  auto fill_all = [&] {
+    std::vector<std::thread> th;
+    uint32_t k = 1;
+    try {
+      for (th.reserve(parts); k < parts; ++k) th.emplace_back(part, k);
+    } catch (...) {  // no more threads: the rest here
+    }
+    part(0);
+    for (; k < parts; ++k) part(k);
+    for (auto& t : th) t.join();
+  };
   std::thread filler;
-  if (n >= 65536)
-    filler = std::thread([&] {
-      const uint32_t parts = std::min(6u, std::max(1u, std::thread::hardware_concurrency() / 2));
-      auto part = [&](uint32_t k) { fill(uint32_t(uint64_t(n) * k / parts), uint32_t(uint64_t(n) * (k + 1) / parts)); };
-      std::vector<std::thread> th;
-      for (uint32_t k = 1; k < parts; ++k) th.emplace_back(part, k);
-      part(0);
-      for (auto& t : th) t.join();
-    });
+  if (parts > 1) {
+    try {
+      filler = std::thread(fill_all);
+    } catch (...) {  // filled after the call instead
+    }
+  }
   const int rc = P.slot0().run_compare(1, false, nullptr);
   if (filler.joinable()) filler.join();
-  else if (!rc) fill(0, n);
+  else if (!rc) fill_all();
   if (rc) return rc;
   const uint32_t queued = P.slot0().err_host.h[2];
   uint32_t c[TC_NCOUNTERS] = {0};

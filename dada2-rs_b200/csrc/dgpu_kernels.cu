@@ -2709,7 +2709,13 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
       const bool stored = __dmul_rn(lam, T.total_reads) > e;  // k_store's rule (src/cluster.rs:379-396)
       if (stored) {
         const double ne = __dmul_rn(lam, double(T.center_reads));
-        if (ne > e) L.pool.e_minmax[g] = ne;
+        if (ne > e) {
+          L.pool.e_minmax[g] = ne;
+          // with several streams the host may start the sample's next call on
+          // another one as soon as it has the posts: the bound is in the
+          // device's memory before they leave
+          if (L.many_slots) __threadfence();
+        }
       }
       const uint32_t bits = R.ham | (uint32_t(R.method) << kPostMethod) | (uint32_t(stored) << kPostStored) |
                             (uint32_t(failed) << kPostError) | (t << kPostTask);
