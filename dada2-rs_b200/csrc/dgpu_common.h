@@ -185,10 +185,30 @@ __host__ __device__ constexpr int strip_rows_per_word(int c) { return c == 1 ? 1
 __host__ __device__ inline size_t strip_plane_bytes(int64_t lmax, int c) {
   return size_t((lmax + 32 + 2 * c) / strip_rows_per_word(c) + 2) * 256;
 }
+// Four bytes per base (two code rows, whose bytes the 2-byte lambda indices take
+// over after the traceback, qualities and transition codes) and the pointer
+// words that stay here. Without the words, which stop at about 461 bases, this
+// is less than either layout it replaces at every length (the row-major one
+// takes five bytes per base), so no pool that those can launch is too long for it:
+// with indices of their own, six bytes a base, blocks passed 227 KB from 9,169 bases on.
 __host__ __device__ inline size_t strip_smem_per_warp(const NwGeom& g) {
   const size_t st = g.strip_smem ? strip_plane_bytes(g.lmax, g.strip_c) : 0;
-  const size_t fi = align16(size_t(g.lmax) * 2);
-  return 2 * align16(size_t(g.lmax) + kStripPad) + 2 * align16(size_t(g.lmax)) + (st > fi ? st : fi);
+  return 2 * align16(size_t(g.lmax) + kStripPad) + 2 * align16(size_t(g.lmax)) + st;
+}
+// The strip aligner's part of a geometry with bands of W diagonals, for pools
+// that strip_takes: the pointer words stay in shared memory while they are
+// small and the block still fits beside the error matrix or the final pass's
+// histograms, 16 x ncol entries per warp.
+constexpr size_t kBlockSmemMax = 226 * 1024;  // 227 KB less the kernels' static arrays
+__host__ __device__ inline size_t strip_block_bytes(const NwGeom& g, int ncol) {
+  const size_t hist = kNwWarps * align16(size_t(16) * size_t(ncol) * 4), err = err_smem_bytes(ncol);
+  return kNwWarps * strip_smem_per_warp(g) + (hist > err ? hist : err);
+}
+inline void strip_geometry(NwGeom& g, int64_t W, int ncol) {
+  g.strip_c = strip_cols(W);
+  g.strip_smem = 1;
+  if (strip_plane_bytes(g.lmax, g.strip_c) > kStripSmemMax || strip_block_bytes(g, ncol) > kBlockSmemMax)
+    g.strip_smem = 0;
 }
 // Bytes of global scratch an alignment warp needs.
 __host__ __device__ inline size_t nw_scratch_bytes(const NwGeom& g) {

@@ -799,8 +799,7 @@ struct Pool {
     geom.strip_c = geom.strip_smem = 0;
     if (rm_possible != vec_possible &&
         strip_takes(lmax, W, vec_possible, kp.match, kp.mismatch, kp.gap, use_homo ? kp.homo_gap : kp.gap)) {
-      geom.strip_c = strip_cols(W);
-      geom.strip_smem = strip_plane_bytes(lmax, geom.strip_c) <= kStripSmemMax ? 1 : 0;
+      strip_geometry(geom, W, kp.ncol);
       geom.forms = geom.strip_c == 1 && !use_homo ? kFormsStrip1 : kFormsStrip;
     }
     const size_t per = std::max<size_t>(nw_scratch_bytes(geom), 16);
@@ -4260,10 +4259,8 @@ int dgpu_align_debug(int device, int which, int npairs, const uint8_t* s1cat, co
   g.rm_scratch = align16(size_t(2 * lmax + 1) * 2 * rm_kbound(g.rm_pairs) * 4);
   g.nwarps = npairs;
   if (lmin >= 2 && end_gap == 0 &&
-      strip_takes(lmax, W, which == 0, kp.match, kp.mismatch, kp.gap, which == 1 ? kp.homo_gap : kp.gap)) {
-    g.strip_c = strip_cols(W);
-    g.strip_smem = strip_plane_bytes(lmax, g.strip_c) <= kStripSmemMax ? 1 : 0;
-  }
+      strip_takes(lmax, W, which == 0, kp.match, kp.mismatch, kp.gap, which == 1 ? kp.homo_gap : kp.gap))
+    strip_geometry(g, W, 1);
   const size_t per = g.strip_c ? strip_plane_bytes(lmax, g.strip_c) : (which == 0 ? g.vec_scratch : g.rm_scratch);
   DBuf<uint8_t> d1, d2, scr, a0, a1;
   DBuf<uint32_t> o1, l1, o2, l2, ao, al, ew;

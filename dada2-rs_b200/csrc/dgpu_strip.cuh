@@ -19,7 +19,7 @@ struct StripSmem {
   uint8_t* qual;    // raw qualities
   uint8_t* tcode;   // per raw position: error-matrix row (see kUnaligned)
   uint2* stage;     // the pointer words, when they stay in shared memory
-  uint16_t* fidx;   // in stage, which is free after the traceback
+  uint16_t* fidx;   // in s1 and s2, which are free once the transition codes are there
 };
 
 __device__ __forceinline__ StripSmem carve_strip(unsigned char* base, const NwGeom& g) {
@@ -30,7 +30,7 @@ __device__ __forceinline__ StripSmem carve_strip(unsigned char* base, const NwGe
   S.qual = base + 2 * ls;
   S.tcode = base + 2 * ls + lq;
   S.stage = reinterpret_cast<uint2*>(base + 2 * ls + 2 * lq);
-  S.fidx = reinterpret_cast<uint16_t*>(S.stage);
+  S.fidx = reinterpret_cast<uint16_t*>(base);
   return S;
 }
 
