@@ -2672,8 +2672,9 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
   // cuts a long pair's latency, the bound of such calls. Wider bands (eight
   // or sixteen groups, G > 1 per warp) keep one warp per pair.
   constexpr bool STRIP = FORMS == kFormsStrip1 || FORMS == kFormsStrip;
-  const bool coop = !STRIP && L.geom.vec_scratch == 0 && kb >= 2 && kb <= kNwWarps && count <= 2u * gridDim.x;
   const bool direct = L.direct != 0;
+  const bool coop = !STRIP && L.geom.vec_scratch == 0 && kb >= 2 && kb <= kNwWarps &&
+                    count <= 2u * uint32_t((direct ? L.geom.late_warps : L.geom.nwarps) / kNwWarps);
   if (blockIdx.x >= count && !direct) return;  // nothing queued for this block
   const size_t err_bytes = err_smem_bytes(kp.ncol);
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -2749,6 +2750,12 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
     if (threadIdx.x == 0) reinterpret_cast<volatile uint32_t*>(L.err_host)[0] = *(volatile uint32_t*)L.err_word;
     if (threadIdx.x < 8) L.queue_counts[threadIdx.x] = 0;
   };
+  auto raw_of = [&](uint32_t slot, uint32_t* task) {
+    const uint32_t item = L.queue_pass[slot];
+    const uint32_t t = find_task(L.task_prefix, L.ntask, item);
+    *task = t;
+    return L.tasks[t].base + (item - L.task_prefix[t]);
+  };
   if constexpr (!STRIP) if (coop) {
     // Thread 0 claims a slot for the CTA and reads the raw's screen distance
     // (which warp 0 overwrites with lambda when the pair is done) into shared
@@ -2761,12 +2768,6 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
     const VecSmem VS0 = carve_vec(w0, L.geom.lmax, L.geom.vec_ncol);
     const RmSmem RS0 = carve_rm(w0, L.geom.lmax, kb);
     uint8_t* scratch0 = L.nw_scratch + size_t(blockIdx.x) * kNwWarps * scr_stride;
-    auto raw_of = [&](uint32_t slot, uint32_t* task) {
-      const uint32_t item = L.queue_pass[slot];
-      const uint32_t t = find_task(L.task_prefix, L.ntask, item);
-      *task = t;
-      return L.tasks[t].base + (item - L.task_prefix[t]);
-    };
     for (;;) {
       if (threadIdx.x == 0) {
         const uint32_t sl = atomicAdd(&L.queue_counts[6], 1u);
@@ -2794,18 +2795,21 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
   // One warp of every block takes a short queue's pairs before any block uses
   // a second, so that the pairs spread over the SMs instead of filling the
   // first blocks (a call with about 740 pairs of 1,450 nt: 0.77 -> 0.43 ms).
-  // After that warps claim queue slots one at a time from a shared cursor
-  // (cleared with the other counters after each call), so pairs of unequal cost -- gapless
-  // against NW, short against long -- and CTAs that become resident late
-  // (when shared memory admits fewer CTAs per SM than the grid assumes) even
-  // out. Results go to each raw's own entries, so the order is free.
+  // The second warp to take one is two warps on: where an SM holds two blocks,
+  // the next one's scheduler already has the other block's first (399 pairs of
+  // 4,000 nt: 1.64 ms in order, 1.48 this way; another first warp in every
+  // block puts four blocks' pairs on one scheduler, late calls of 1,500 nt
+  // 165 -> 235 us). After that warps claim queue slots one at a time from a
+  // shared cursor (cleared with the other counters after each call), so pairs
+  // of unequal cost -- gapless against NW, short against long -- even out.
+  // Results go to each raw's own entries, so the order is free.
   auto each_pair = [&](auto&& align) {
     // the first slot is the warp's own, the rest come from the cursor
-    for (uint32_t slot = uint32_t(wib) * gridDim.x + blockIdx.x; slot < count;) {
-      const uint32_t item = L.queue_pass[slot];
-      const uint32_t t = find_task(L.task_prefix, L.ntask, item);
+    const uint32_t turn = uint32_t(wib & 1) * 2 + uint32_t(wib >> 1);
+    for (uint32_t slot = turn * gridDim.x + blockIdx.x; slot < count;) {
+      uint32_t t;
+      const uint32_t g = raw_of(slot, &t);
       const TaskDev T = L.tasks[t];
-      const uint32_t g = T.base + (item - L.task_prefix[t]);
       const double e = direct ? L.pool.e_minmax[g] : 0.0;
       finish(align(g, T.center), g, t, T, slot, e);
       if (lane == 0) slot = kNwWarps * gridDim.x + atomicAdd(&L.queue_counts[6], 1u);
@@ -3143,15 +3147,24 @@ uint32_t compare_screen_chunk(uint32_t total, uint32_t screen_blocks_per_sm, uin
 
 // The k_align instance for the forms a launch can reach, with its attributes
 // set once per device (dynamic shared memory above 48 KB, the largest
-// carveout so that kAlignCtasPerSm CTAs fit beside each other).
+// carveout so that kAlignCtasPerSm CTAs fit beside each other), and the blocks
+// of it that fit the device at once.
 template <class Tb>
-static void (*align_kernel(const CompareLaunch& L, size_t smem))(CompareLaunch, Tb) {
+struct AlignKernel {
+  void (*fn)(CompareLaunch, Tb);
+  size_t smem;
+  uint32_t resident;
+};
+template <class Tb>
+static AlignKernel<Tb> align_kernel(const CompareLaunch& L) {
   static void (*const forms[4])(CompareLaunch, Tb) = {k_align<kFormsAll, Tb>, k_align<kFormsStrip1, Tb>,
                                                       k_align<kFormsRm, Tb>, k_align<kFormsStrip, Tb>};
   const int fi = L.geom.forms;
+  const size_t smem = err_smem_bytes(L.kp.ncol) + size_t(kNwWarps) * align_smem_per_warp(L.geom);
   void (*kalign)(CompareLaunch, Tb) = forms[fi];
   static std::atomic<int> limit[4][64];
   static std::atomic<uint64_t> carved[4];
+  static std::atomic<uint64_t> fits[4][64];  // of the latest size: bytes << 8 | blocks per SM
   int dev = 0;
   cudaGetDevice(&dev);
   std::atomic<int>& lim = limit[fi][dev & 63];
@@ -3164,7 +3177,17 @@ static void (*align_kernel(const CompareLaunch& L, size_t smem))(CompareLaunch, 
     cudaFuncSetAttribute(kalign, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     carved[fi].fetch_or(bit);
   }
-  return kalign;
+  uint64_t f = fits[fi][dev & 63].load(std::memory_order_relaxed);
+  if (f >> 8 != smem) {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kalign, kNwWarps * 32, smem) != cudaSuccess) {
+      (void)cudaGetLastError();  // the launch will tell
+      n = kAlignCtasPerSm;
+    }
+    f = uint64_t(smem) << 8 | uint64_t(std::min(std::max(n, 1), kAlignCtasPerSm));
+    fits[fi][dev & 63].store(f, std::memory_order_relaxed);
+  }
+  return {kalign, smem, uint32_t(f & 255u) * uint32_t(sm_count())};
 }
 
 // The launch sequence of one compare: k_pivot_dots (pivot_blocks > 0), the
@@ -3173,7 +3196,7 @@ static void (*align_kernel(const CompareLaunch& L, size_t smem))(CompareLaunch, 
 template <class Tb>
 static void launch_chain(const CompareLaunch& L, const Tb& tb, cudaStream_t st, cudaEvent_t* ev,
                          uint32_t screen_blocks, uint32_t pivot_blocks, uint32_t store_grid,
-                         void (*kalign)(CompareLaunch, Tb), size_t asmem) {
+                         const AlignKernel<Tb>& align) {
   if (ev) cudaEventRecord(ev[0], st);
   if (pivot_blocks > 0) {
     switch (L.kp.kmer_size) {
@@ -3212,10 +3235,14 @@ static void launch_chain(const CompareLaunch& L, const Tb& tb, cudaStream_t st, 
   // (a call of 24,908 pairs of 250 nt: 0.97 ms with two blocks per SM, 0.53 with
   // four).
   const bool late = L.do_store && store_grid == 0;
-  cfg.gridDim = dim3(late ? L.geom.late_warps / kNwWarps : L.geom.nwarps / kNwWarps);
+  // No more blocks than fit at once: each takes its first pairs by its index,
+  // and those of a block that waits for another's end come a whole pair late
+  // (399 pairs of 4,000 nt, two blocks per SM: 2.82 ms, now 1.48; 600 of
+  // 3,400 nt, three per SM: 0.78 and 0.44).
+  cfg.gridDim = dim3(std::min(uint32_t(late ? L.geom.late_warps : L.geom.nwarps) / kNwWarps, align.resident));
   cfg.blockDim = dim3(kNwWarps * 32);
-  cfg.dynamicSmemBytes = asmem;
-  cudaLaunchKernelEx(&cfg, kalign, L, tb);
+  cfg.dynamicSmemBytes = align.smem;
+  cudaLaunchKernelEx(&cfg, align.fn, L, tb);
   if (ev) cudaEventRecord(ev[2], st);
   if (store_grid > 0) {
     cfg.gridDim = dim3(store_grid);
@@ -3245,21 +3272,19 @@ void launch_compare(const CompareLaunch& L0, cudaStream_t st, cudaEvent_t* ev) {
   const uint32_t pb = (L.cdot_ready && L.total_cl > 0 && L.kp.kmer_size <= 7)
                           ? std::min<uint32_t>((L.total_cl + 7) / 8, uint32_t(sms) * 8u)
                           : 0u;
-  const size_t asm_ = err_smem_bytes(L.kp.ncol) + size_t(kNwWarps) * align_smem_per_warp(L.geom);
   const uint32_t store = L.do_store && !L.direct ? L.nstore_blocks : 0u;
-  if (L.tables) launch_chain(L, *L.tables, st, ev, blocks, pb, store, align_kernel<CallTables>(L, asm_), asm_);
-  else launch_chain(L, NoTables{}, st, ev, blocks, pb, store, align_kernel<NoTables>(L, asm_), asm_);
+  if (L.tables) launch_chain(L, *L.tables, st, ev, blocks, pb, store, align_kernel<CallTables>(L));
+  else launch_chain(L, NoTables{}, st, ev, blocks, pb, store, align_kernel<NoTables>(L));
 }
 
 int capture_compare_graph(const CompareLaunch& L, cudaStream_t st, uint32_t screen_grid, bool pivot_dots,
                           uint32_t store_grid, cudaGraph_t* out) {
   const int sms = sm_count();
-  const size_t asm_ = err_smem_bytes(L.kp.ncol) + size_t(kNwWarps) * align_smem_per_warp(L.geom);
-  void (*kalign)(CompareLaunch, NoTables) = align_kernel<NoTables>(L, asm_);  // attributes before the capture
+  const AlignKernel<NoTables> align = align_kernel<NoTables>(L);  // attributes before the capture
   cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return int(e);
   launch_chain(L, NoTables{}, st, nullptr, screen_grid, pivot_dots && L.kp.kmer_size <= 7 ? uint32_t(sms) * 8u : 0u,
-               store_grid, kalign, asm_);
+               store_grid, align);
   cudaGraph_t g = nullptr;
   e = cudaStreamEndCapture(st, &g);
   if (e != cudaSuccess) {
