@@ -118,6 +118,11 @@ constexpr int32_t kFormsAll = 0;   // every form
 constexpr int32_t kFormsStrip1 = 1;  // gapless and the strip aligner, one diagonal per strip, no homopolymer gaps
 constexpr int32_t kFormsRm = 2;    // gapless and the row-major forms
 constexpr int32_t kFormsStrip = 3;   // gapless and the strip aligner, up to four diagonals per strip
+// Gapless and the vectorized forms, for pools beyond the strip aligner's rule
+// (more than 248 diagonals, scores past its bounds) with nothing row-major.
+// Without the row-major code nothing spills: 4,000 uniques of 150 nt at
+// mismatch -220 0.25 -> 0.23 ms a call, of 1,000 nt at band 140 8.7 -> 7.9 ms.
+constexpr int32_t kFormsVec = 4;
 
 // ---- shared-memory carving, used by kernels and by the host sizing code ----
 constexpr int kScreenWarps = 8;   // warps per screen CTA

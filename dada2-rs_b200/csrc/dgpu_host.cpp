@@ -795,7 +795,7 @@ struct Pool {
     geom.late_warps = sms * tuning_for(lmax).align_ctas_per_sm * kNwWarps;
     // the forms k_align can reach: the strip aligner alone when it takes every
     // pair (see strip_takes), one diagonal per strip when no pair needs more
-    geom.forms = rm_possible && !vec_possible ? kFormsRm : kFormsAll;
+    geom.forms = !vec_possible ? kFormsRm : (rm_possible ? kFormsAll : kFormsVec);
     geom.strip_c = geom.strip_smem = 0;
     if (rm_possible != vec_possible &&
         strip_takes(lmax, W, vec_possible, kp.match, kp.mismatch, kp.gap, use_homo ? kp.homo_gap : kp.gap)) {

@@ -2598,7 +2598,7 @@ __device__ __forceinline__ PairResult align_pair(int lane, const KParams& kp, co
   const uint8_t* qg = pool.qual ? pool.qual + pool.off[g] : nullptr;
   const bool use_homo = kp.homo_gap != kp.gap && kp.homo_gap <= 0;
   const bool rm_pair = use_homo || !kp.vectorized || lc > 3500 || lg > 3500;
-  const bool rm = FORMS == kFormsRm ? true : rm_pair;
+  const bool rm = FORMS == kFormsRm ? true : (FORMS == kFormsVec ? false : rm_pair);
   if (rm != rm_pair) {
     if (lane == 0) atomicOr(err_word, DERR_UNSUPPORTED);
     return PairResult{false, AM_NONE, 0u, lg, VS.tcode, VS.fidx, qg};
@@ -2628,7 +2628,7 @@ __device__ __forceinline__ PairResult align_pair(int lane, const KParams& kp, co
     R.ok = vec_align_any(lane, sc, lc, sg, lg, int16_t(kp.match), int16_t(kp.mismatch), int16_t(kp.gap), 0, kp.band,
                          VS, scratch, geom.vec_ncol, geom.vec_nrow, &ham, err_word, nullptr, nullptr, nullptr, true);
     R.method = AM_VECTORIZED;
-  } else {
+  } else if constexpr (FORMS != kFormsVec) {
     if (COOP)
       R.ok = rm_dispatch_coop(lane, wib, sc, lc, sg, lg, kp, use_homo, kb, RS, reinterpret_cast<uint32_t*>(scratch),
                               &ham, err_word, xch);
@@ -2673,7 +2673,8 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
   // or sixteen groups, G > 1 per warp) keep one warp per pair.
   constexpr bool STRIP = FORMS == kFormsStrip1 || FORMS == kFormsStrip;
   const bool direct = L.direct != 0;
-  const bool coop = !STRIP && L.geom.vec_scratch == 0 && kb >= 2 && kb <= kNwWarps &&
+  constexpr bool COOP = FORMS == kFormsRm;
+  const bool coop = COOP && L.geom.vec_scratch == 0 && kb >= 2 && kb <= kNwWarps &&
                     count <= 2u * uint32_t((direct ? L.geom.late_warps : L.geom.nwarps) / kNwWarps);
   if (blockIdx.x >= count && !direct) return;  // nothing queued for this block
   const size_t err_bytes = err_smem_bytes(kp.ncol);
@@ -2756,7 +2757,7 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
     *task = t;
     return L.tasks[t].base + (item - L.task_prefix[t]);
   };
-  if constexpr (!STRIP) if (coop) {
+  if constexpr (COOP) if (coop) {
     // Thread 0 claims a slot for the CTA and reads the raw's screen distance
     // (which warp 0 overwrites with lambda when the pair is done) into shared
     // memory, so every warp takes the same branches through the pair and the
@@ -2808,10 +2809,18 @@ __global__ void __launch_bounds__(kNwWarps * 32, kAlignCtasPerSm) k_align(Compar
     const uint32_t turn = uint32_t(wib & 1) * 2 + uint32_t(wib >> 1);
     for (uint32_t slot = turn * gridDim.x + blockIdx.x; slot < count;) {
       uint32_t t;
-      const uint32_t g = raw_of(slot, &t);
-      const TaskDev T = L.tasks[t];
-      const double e = direct ? L.pool.e_minmax[g] : 0.0;
-      finish(align(g, T.center), g, t, T, slot, e);
+      uint32_t g = raw_of(slot, &t);
+      if constexpr (STRIP) {
+        const TaskDev T = L.tasks[t];
+        const double e = direct ? L.pool.e_minmax[g] : 0.0;
+        finish(align(g, T.center), g, t, T, slot, e);
+      } else {
+        // these aligners need every register and more: the pair's raw, task
+        // and bound are read anew after them
+        const PairResult R = align(g, L.tasks[t].center);
+        g = raw_of(slot, &t);
+        finish(R, g, t, L.tasks[t], slot, direct ? L.pool.e_minmax[g] : 0.0);
+      }
       if (lane == 0) slot = kNwWarps * gridDim.x + atomicAdd(&L.queue_counts[6], 1u);
       slot = __shfl_sync(FULL, slot, 0);
     }
@@ -3157,14 +3166,15 @@ struct AlignKernel {
 };
 template <class Tb>
 static AlignKernel<Tb> align_kernel(const CompareLaunch& L) {
-  static void (*const forms[4])(CompareLaunch, Tb) = {k_align<kFormsAll, Tb>, k_align<kFormsStrip1, Tb>,
-                                                      k_align<kFormsRm, Tb>, k_align<kFormsStrip, Tb>};
+  static void (*const forms[5])(CompareLaunch, Tb) = {k_align<kFormsAll, Tb>, k_align<kFormsStrip1, Tb>,
+                                                      k_align<kFormsRm, Tb>, k_align<kFormsStrip, Tb>,
+                                                      k_align<kFormsVec, Tb>};
   const int fi = L.geom.forms;
   const size_t smem = err_smem_bytes(L.kp.ncol) + size_t(kNwWarps) * align_smem_per_warp(L.geom);
   void (*kalign)(CompareLaunch, Tb) = forms[fi];
-  static std::atomic<int> limit[4][64];
-  static std::atomic<uint64_t> carved[4];
-  static std::atomic<uint64_t> fits[4][64];  // of the latest size: bytes << 8 | blocks per SM
+  static std::atomic<int> limit[5][64];
+  static std::atomic<uint64_t> carved[5];
+  static std::atomic<uint64_t> fits[5][64];  // of the latest size: bytes << 8 | blocks per SM
   int dev = 0;
   cudaGetDevice(&dev);
   std::atomic<int>& lim = limit[fi][dev & 63];
