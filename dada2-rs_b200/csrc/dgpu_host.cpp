@@ -791,8 +791,6 @@ struct Pool {
     // (at most 4 groups) for the register form
     geom.vec_scratch = vec_possible ? align16(size_t(geom.vec_nrow) * std::max<size_t>(size_t(geom.vec_ncol), 32)) : 0;
     geom.rm_scratch = rm_possible ? align16(size_t(2 * lmax + 1) * 2 * kb * 4) : 0;
-    geom.nwarps = sms * kAlignCtasPerSm * kNwWarps;
-    geom.late_warps = sms * tuning_for(lmax).align_ctas_per_sm * kNwWarps;
     // the forms k_align can reach: the strip aligner alone when it takes every
     // pair (see strip_takes), one diagonal per strip when no pair needs more
     geom.forms = !vec_possible ? kFormsRm : (rm_possible ? kFormsAll : kFormsVec);
@@ -803,6 +801,14 @@ struct Pool {
       geom.forms = geom.strip_c == 1 && !use_homo ? kFormsStrip1 : kFormsStrip;
     }
     const size_t per = std::max<size_t>(nw_scratch_bytes(geom), 16);
+    // A call that aligns most uniques wants four blocks per SM (launch_chain);
+    // their scratch, one piece per warp and launch slot, stays below 2 GB or at
+    // the tuned number's: bands without a bound at 3,500 nt take 58 GB in full,
+    // and a tuning to fewer blocks is what makes them fit. At the committed
+    // tuning nothing is that large below 600 nt.
+    geom.late_warps = sms * tuning_for(lmax).align_ctas_per_sm * kNwWarps;
+    geom.nwarps = sms * kAlignCtasPerSm * kNwWarps;
+    if (per * size_t(geom.nwarps) > (size_t(2) << 30)) geom.nwarps = geom.late_warps;
     slots.clear();
     for (int k = 0; k < nslots; ++k) {
       slots.emplace_back(new Slot);
