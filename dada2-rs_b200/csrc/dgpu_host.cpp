@@ -588,11 +588,12 @@ struct Slot {
   template <class F>
   void for_each_stored(uint32_t t, F&& f) const;
   void task_counters(uint32_t t, uint32_t* out) const;
-  // whether a call of ntask tasks can store directly
-  bool direct_fits(uint32_t ntask) const;
+  // whether a call of ntask tasks that is expected to queue `pairs` can store directly
+  bool direct_fits(uint32_t ntask, uint64_t pairs) const;
   // may_direct: direct_fits, no raw of the tasks has a negative e_minmax, and few comps are
   // expected (CompareLaunch::direct)
-  int run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_direct = false);
+  int run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_direct = false,
+                  Clock::time_point t_call = Clock::now());
   // whether every post of the latest direct call has come
   bool posts_here(uint32_t ntask);
   // the call's counters and comps from its posts; false: it queued more pairs
@@ -861,8 +862,12 @@ static double f64_of(uint64_t bits) {
   return d;
 }
 
-bool Slot::direct_fits(uint32_t ntask) const {
-  return P->kp.use_kmers && !P->kp.lambda32 && ntask <= uint32_t(kScreenSmemTasks);
+// Pairs a launch may be expected to queue and still store directly: a quarter of
+// the posts is left for calls that align more than their samples' last ones.
+constexpr uint32_t kPostExpect = kPostMax / 4 * 3;
+
+bool Slot::direct_fits(uint32_t ntask, uint64_t pairs) const {
+  return P->kp.use_kmers && !P->kp.lambda32 && ntask <= uint32_t(kScreenSmemTasks) && pairs <= kPostExpect;
 }
 
 // Stored comps of task t (latest launch), in ascending raw order.
@@ -946,8 +951,7 @@ bool Slot::read_posts(uint32_t ntask) {
 // Launches one compare over `ntask` tasks already in task_stage; waits for it.
 // The launch's tables go up in one copy; with the store, the error flags come
 // back through mapped memory and the queue counters are rearmed on the device.
-int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_direct) {
-  const auto t_call = Clock::now();
+int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_direct, Clock::time_point t_call) {
   TRY(ensure_tasks(ntask));
   const Pool& Q = *P;
   direct = may_direct && do_store;
@@ -1146,6 +1150,9 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_di
   CUDA_TRY(q);
   const auto t1 = Clock::now();
   if (wait_s) *wait_s += secs(t0, t1);
+  // a direct call with more pairs than it posts aligned none and is made again:
+  // its launches count, the call itself counts once
+  const bool again = direct && posts_here(ntask) && uint32_t(post.h[0]) > kPostMax;
   {
     float ms[3] = {0, 0, 0};
     if (timing)
@@ -1160,27 +1167,29 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_di
     S.launches[1] += 1;
     S.launches[2] += 1;
     if (do_store && !direct) S.launches[3] += 1;
-    for (int k = 0; k < 3; ++k) S.ms[k + 1] += ms[k];
-    S.rounds += 1;
-    S.compares += total;
-    S.screened += screened;
-    // algorithmic screen bytes: the 4^k profile of every raw whose profile the
-    // screen read (screened raws less those the pivot bound excluded), or
-    // for k = 8 the sparse list of every screened raw (3 bytes per present
-    // k-mer, at most L - k + 1); 16 B of metadata per compare, 8 more for the
-    // pivot when the loop keeps pivots; and both profiles of each center dot
-    const uint64_t prof = Q.kp.kmer_size >= 8 ? uint64_t(3) * (Q.lmax - uint32_t(Q.kp.kmer_size) + 1)
-                                              : (uint64_t(1) << (2 * Q.kp.kmer_size));
-    const uint64_t nread = Q.kp.kmer_size >= 8 ? screened : direct ? uint64_t(uint32_t(post.h[1])) : uint64_t(err_host.h[1]);
-    const uint64_t sb = nread * prof + uint64_t(total) * (pivot ? 24u : 16u) +
-                        (cdot_ready ? uint64_t(total_cl) * 2u * prof : 0u);
-    S.screen_bytes += sb;
-    if (timing) {
-      S.timed_rounds += 1;
-      S.timed_screen_bytes += sb;
-      S.timed_compares += total;
+    if (!again) {
+      for (int k = 0; k < 3; ++k) S.ms[k + 1] += ms[k];
+      S.rounds += 1;
+      S.compares += total;
+      S.screened += screened;
+      // algorithmic screen bytes: the 4^k profile of every raw whose profile the
+      // screen read (screened raws less those the pivot bound excluded), or
+      // for k = 8 the sparse list of every screened raw (3 bytes per present
+      // k-mer, at most L - k + 1); 16 B of metadata per compare, 8 more for the
+      // pivot when the loop keeps pivots; and both profiles of each center dot
+      const uint64_t prof = Q.kp.kmer_size >= 8 ? uint64_t(3) * (Q.lmax - uint32_t(Q.kp.kmer_size) + 1)
+                                                : (uint64_t(1) << (2 * Q.kp.kmer_size));
+      const uint64_t nread = Q.kp.kmer_size >= 8 ? screened : direct ? uint64_t(uint32_t(post.h[1])) : uint64_t(err_host.h[1]);
+      const uint64_t sb = nread * prof + uint64_t(total) * (pivot ? 24u : 16u) +
+                          (cdot_ready ? uint64_t(total_cl) * 2u * prof : 0u);
+      S.screen_bytes += sb;
+      if (timing) {
+        S.timed_rounds += 1;
+        S.timed_screen_bytes += sb;
+        S.timed_compares += total;
+      }
+      if (g_stats.round_ms.size() < (size_t(1) << 20)) g_stats.round_ms.push_back(1e3 * secs(t_call, t1));
     }
-    if (g_stats.round_ms.size() < (size_t(1) << 20)) g_stats.round_ms.push_back(1e3 * secs(t_call, t1));
   }
   const uint32_t ew = *reinterpret_cast<volatile uint32_t*>(err_host.h);
   if (ew) {
@@ -1198,7 +1207,7 @@ int Slot::run_compare(uint32_t ntask, bool do_store, double* wait_s, bool may_di
   }
   if (direct && !posts_here(ntask)) return fail(DGPU_E_DEVICE, "device error: a compare call ended without its posts");
   // too many pairs for a direct call, none of which it aligned
-  if (direct && !read_posts(ntask)) return run_compare(ntask, do_store, wait_s, false);
+  if (direct && !read_posts(ntask)) return run_compare(ntask, do_store, wait_s, false, t_call);
   return 0;
 }
 
@@ -1459,9 +1468,11 @@ struct SampleState {
   RunStats stats;
   bool lock_dirty = false, done = false;
   // The next compare call may store directly: every raw's e_minmax is set, and
-  // the last call aligned few pairs (clusters come largest first, so the next
-  // aligns about as few; more than kPostMax would make the call twice).
-  bool few_pairs = false, e_set = false;
+  // the pairs the last call aligned leave room among the launch's (clusters come
+  // largest first, so the next call aligns about as many; more than kPostMax in
+  // a launch would make it twice).
+  uint32_t last_pairs = UINT32_MAX;
+  bool e_set = false;
   std::vector<uint32_t> lock_new;  // raws locked since the last call, up to one past kLockListMax
   int64_t pending = -1;  // cluster whose compare is queued
   // shuffle carry (src/cluster.rs:848-866)
@@ -1706,7 +1717,7 @@ struct SampleState {
     const uint32_t ns = ctr[TC_STORED];
     // a direct call's counters have TC_UNSET 0 and follow one that had
     e_set = ctr[TC_UNSET] == 0;
-    few_pairs = ctr[TC_ALIGNED] < kPostMax / 4;
+    last_pairs = ctr[TC_ALIGNED];
     nalign += ctr[TC_SCREENED];
     nshroud += ctr[TC_SHROUD];
     stats.compare_calls++;
@@ -3086,13 +3097,16 @@ static int run_samples(Pool& P, std::vector<SampleState>& S, const dgpu_align_pa
           for (size_t sidx : batch) S[sidx].stats.t_slot_wait += secs(S[sidx].stats.t_mark, now);
         }
         int r = L.ensure_tasks(uint32_t(batch.size()));
-        bool direct = L.direct_fits(uint32_t(batch.size()));
+        bool direct = true;
+        uint64_t pairs = 0;
         for (size_t a = 0; a < batch.size() && !r; ++a) {
           SampleState& ss = S[batch[a]];
           const size_t ci = size_t(ss.pending);
           L.task_stage.h[a] = ss.task_for(ci, ci == 0 ? 1.0 : ap.kdist_cutoff);  // init_params, src/dada.rs:835-838
-          direct = direct && ss.e_set && ss.few_pairs;
+          direct = direct && ss.e_set && ss.last_pairs < kPostMax / 4;
+          pairs += ss.last_pairs;
         }
+        direct = direct && L.direct_fits(uint32_t(batch.size()), pairs);
         // locks set since a sample's last call: the direct call's screen enters
         // a short list of them itself; else the sample's flags are copied
         L.lock_list.clear();

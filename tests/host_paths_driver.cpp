@@ -66,9 +66,26 @@ static int geometry() {
   return 0;
 }
 
+// Which launches may store directly: the pairs that all of a launch's samples
+// expect together have to fit the posts.
+static int direct_room() {
+  Pool* P = new Pool;
+  P->kp.use_kmers = 1;
+  Slot* L = new Slot;
+  L->P = P;
+  if (int r = check(1, L->direct_fits(8, 8 * 1000) == false)) return r;  // each sample's would, all eight's do not
+  if (int r = check(2, L->direct_fits(8, 8 * 300) == true)) return r;
+  if (int r = check(3, L->direct_fits(1, 1000) == true)) return r;
+  if (int r = check(4, L->direct_fits(kScreenSmemTasks + 1, 10) == false)) return r;
+  if (int r = check(5, kPostExpect < kPostMax && L->direct_fits(2, kPostExpect) && !L->direct_fits(2, kPostExpect + 1)))
+    return r;
+  P->kp.lambda32 = 1;
+  return check(6, L->direct_fits(1, 10) == false);
+}
+
 int main(int argc, char** argv) {
   const std::string what = argc > 1 ? argv[1] : "";
-  const int r = what == "geometry" ? geometry() : 99;
+  const int r = what == "geometry" ? geometry() : what == "direct_room" ? direct_room() : 99;
   if (r == 0) std::printf("ok\n");
   return r;
 }

@@ -29,3 +29,7 @@ def run(driver, what):
 
 def test_scratch_of_the_resident_warps_is_bounded_by_the_tuning(driver):
     run(driver, "geometry")
+
+
+def test_direct_calls_are_sized_by_the_launch(driver):
+    run(driver, "direct_room")
