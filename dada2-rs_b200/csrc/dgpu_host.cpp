@@ -3903,15 +3903,20 @@ int dgpu_compare(dgpu_ctx* ctx, int center, double kdist_cutoff, int greedy, dou
     for (; k < parts; ++k) part(k);
     for (auto& t : th) t.join();
   };
-  std::thread filler;
+  struct Filler {
+    std::thread t;
+    ~Filler() {
+      if (t.joinable()) t.join();  // also when the call below throws
+    }
+  } filler;
   if (parts > 1) {
     try {
-      filler = std::thread(fill_all);
+      filler.t = std::thread(fill_all);
     } catch (...) {  // filled after the call instead
     }
   }
   const int rc = P.slot0().run_compare(1, false, nullptr);
-  if (filler.joinable()) filler.join();
+  if (filler.t.joinable()) filler.t.join();
   else if (!rc) fill_all();
   if (rc) return rc;
   const uint32_t queued = P.slot0().err_host.h[2];

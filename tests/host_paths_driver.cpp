@@ -26,6 +26,17 @@ void launch_align_debug(int, const uint8_t*, const uint32_t*, const uint32_t*, c
 
 using namespace dgpu;
 
+// operator new throws on this thread once `left` allocations have passed
+static thread_local long left = -1;
+void* operator new(size_t n) {
+  if (left == 0) throw std::bad_alloc();
+  if (left > 0) --left;
+  if (void* p = std::malloc(n ? n : 1)) return p;
+  throw std::bad_alloc();
+}
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, size_t) noexcept { std::free(p); }
+
 static int check(int no, bool ok) {
   if (!ok) std::printf("check %d failed\n", no);
   return ok ? 0 : no;
@@ -83,9 +94,49 @@ static int direct_room() {
   return check(6, L->direct_fits(1, 10) == false);
 }
 
+// A large map call fills its outputs on other threads; whatever allocation
+// fails meanwhile, the call ends with an error or the exception, not with the
+// program. (Here it ends where it asks for pinned memory at the latest.)
+static int compare_without_memory() {
+  const uint32_t n = 200000;
+  dgpu_ctx* ctx = new dgpu_ctx;  // never freed: its buffers are not
+  ctx->uploaded = true;
+  ctx->reads.assign(n, 1u);
+  ctx->total_reads = n;
+  Pool& P = ctx->pool;
+  P.nraw = n;
+  P.kp.use_kmers = 1;
+  P.kp.kmer_size = 5;
+  P.lock_host.h = static_cast<uint8_t*>(std::calloc(n, 1));
+  P.slots.emplace_back(new Slot);
+  Slot& L = P.slot0();
+  L.P = &P;
+  L.ntask_cap = 1;
+  L.task_stage.h = static_cast<TaskDev*>(std::calloc(1, sizeof(TaskDev)));
+  std::vector<double> lam(n);
+  std::vector<uint32_t> ham(n);
+  std::vector<uint8_t> skipped(n);
+  int threw = 0;
+  for (long allowed = 0; allowed < 24; ++allowed) {
+    int rc = 1;
+    try {
+      left = allowed;
+      rc = dgpu_compare(ctx, 0, 0.42, 1, lam.data(), ham.data(), skipped.data(), nullptr);
+    } catch (const std::bad_alloc&) {
+      ++threw;
+    }
+    left = -1;
+    if (int r = check(1, rc != 0)) return r;
+    std::vector<uint32_t>().swap(L.task_blk0);  // as before the first call
+  }
+  return check(2, threw > 0);
+}
+
 int main(int argc, char** argv) {
   const std::string what = argc > 1 ? argv[1] : "";
-  const int r = what == "geometry" ? geometry() : what == "direct_room" ? direct_room() : 99;
+  const int r = what == "geometry" ? geometry() : what == "direct_room" ? direct_room()
+                : what == "compare_without_memory" ? compare_without_memory()
+                                                   : 99;
   if (r == 0) std::printf("ok\n");
   return r;
 }

@@ -33,3 +33,7 @@ def test_scratch_of_the_resident_warps_is_bounded_by_the_tuning(driver):
 
 def test_direct_calls_are_sized_by_the_launch(driver):
     run(driver, "direct_room")
+
+
+def test_map_call_survives_a_failed_allocation(driver):
+    run(driver, "compare_without_memory")
