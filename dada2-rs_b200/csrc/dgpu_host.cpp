@@ -767,6 +767,10 @@ struct Pool {
   // Per-run device state: every e_minmax back to -999 (B::new,
   // src/containers.rs:342) and no raw with a pivot yet.
   int reset_e_minmax() {
+    // the host goes on once it has a direct call's posts: its last writes to the
+    // bounds may still be on their way, on the slot's own stream
+    for (auto& L : slots)
+      if (L->st) CUDA_TRY(cudaStreamSynchronize(L->st));
     launch_fill_f64(e_minmax.p, nraw, -999.0, st);
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaMemsetAsync(piv_cl.p, 0xff, piv_cl.n * 4, st));
