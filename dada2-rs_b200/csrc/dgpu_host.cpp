@@ -4290,6 +4290,15 @@ int dgpu_align_debug(int device, int which, int npairs, const uint8_t* s1cat, co
   if (lmin >= 2 && end_gap == 0 &&
       strip_takes(lmax, W, which == 0, kp.match, kp.mismatch, kp.gap, which == 1 ? kp.homo_gap : kp.gap))
     strip_geometry(g, W, 1);
+  // the strip aligner keeps flags beside 4-bit codes, as the row-major forms do;
+  // the vectorized ones hand back any byte
+  if (which == 0 && g.strip_c) {
+    auto wide = [](uint8_t c) { return c > 15; };
+    for (int t = 0; t < npairs && g.strip_c; ++t)
+      if (std::any_of(s1cat + off1[t], s1cat + off1[t] + len1[t], wide) ||
+          std::any_of(s2cat + off2[t], s2cat + off2[t] + len2[t], wide))
+        g.strip_c = g.strip_smem = 0;
+  }
   const size_t per = g.strip_c ? strip_plane_bytes(lmax, g.strip_c) : (which == 0 ? g.vec_scratch : g.rm_scratch);
   DBuf<uint8_t> d1, d2, scr, a0, a1;
   DBuf<uint32_t> o1, l1, o2, l2, ao, al, ew;
