@@ -3076,7 +3076,7 @@ __global__ void __launch_bounds__(kStoreThreads) k_store(CompareLaunch Lp) {
 // comp arrays (comp_ham with the aligner above kPostMethod); every other raw's
 // outcome follows from the host's own reads and locks. A call over 400,000
 // uniques moves 0.4 MB for its 28,000 pairs, not the 5.2 MB of every raw's
-// entries. Its first block rearms the queue, as k_store's does.
+// entries. Its last block rearms the queue.
 template <class Tb>
 __global__ void __launch_bounds__(256) k_collect(CompareLaunch Lp, const __grid_constant__ Tb tb) {
   CompareLaunch L = Lp;
@@ -3174,7 +3174,7 @@ static AlignKernel<Tb> align_kernel(const CompareLaunch& L) {
   void (*kalign)(CompareLaunch, Tb) = forms[fi];
   static std::atomic<int> limit[5][64];
   static std::atomic<uint64_t> carved[5];
-  static std::atomic<uint64_t> fits[5][64];  // of the latest size: bytes << 8 | blocks per SM
+  static std::atomic<uint64_t> fits[5][64][16];  // sizes met: bytes << 8 | blocks per SM
   int dev = 0;
   cudaGetDevice(&dev);
   std::atomic<int>& lim = limit[fi][dev & 63];
@@ -3187,7 +3187,8 @@ static AlignKernel<Tb> align_kernel(const CompareLaunch& L) {
     cudaFuncSetAttribute(kalign, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     carved[fi].fetch_or(bit);
   }
-  uint64_t f = fits[fi][dev & 63].load(std::memory_order_relaxed);
+  std::atomic<uint64_t>& fit = fits[fi][dev & 63][(smem >> 4) & 15];
+  uint64_t f = fit.load(std::memory_order_relaxed);
   if (f >> 8 != smem) {
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kalign, kNwWarps * 32, smem) != cudaSuccess) {
@@ -3195,7 +3196,7 @@ static AlignKernel<Tb> align_kernel(const CompareLaunch& L) {
       n = kAlignCtasPerSm;
     }
     f = uint64_t(smem) << 8 | uint64_t(std::min(std::max(n, 1), kAlignCtasPerSm));
-    fits[fi][dev & 63].store(f, std::memory_order_relaxed);
+    fit.store(f, std::memory_order_relaxed);
   }
   return {kalign, smem, uint32_t(f & 255u) * uint32_t(sm_count())};
 }
