@@ -256,7 +256,8 @@ int dgpu_service_submit(dgpu_service* s, int nraw, const char* seqs, const uint3
   const uint64_t total = r->total;
   r->cls = length_class(lmax);
   // device bytes while served: codes and qualities, the k-mer screen, per-raw
-  // state, and the aligners' per-warp pointer scratch of its batch
+  // state, and the aligners' pointer scratch of its batch (about what six launch
+  // slots of the strip aligner take at 1,550 nt; up to 461 nt they take none)
   const int k = s->params.align.kmer_size;
   const uint64_t profile = k >= 8 ? 3 * uint64_t(lmax) : (uint64_t(1) << (2 * k));
   r->footprint = 2 * total + uint64_t(r->n) * (profile + 64) + uint64_t(2 * lmax + 1) * 32 * 2368 * 3;

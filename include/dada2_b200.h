@@ -232,7 +232,8 @@ int dgpu_cache_release(int device, uint64_t* freed);
  * samples_per_launch   most samples one compare launch serves, 1..4096
  * dedicated_slots      slots reserved for the samples with the longest chains, 0..7
  * align_ctas_per_sm    resident CTAs of a late call's alignment kernel per SM (4 pairs
- *                      each), 1..4; a call that aligns most uniques takes 4
+ *                      each), 1..4; a call that aligns most uniques takes 4 unless its
+ *                      scratch would pass 2 GB per launch slot
  * screen_chunk_max     largest run of (center, unique) items one screen warp takes, 16 or 32
  * screen_blocks_per_sm screen blocks per SM in its single wave, 1..4
  * pivot_min_items      compare launches of at least this many (center, unique) items
